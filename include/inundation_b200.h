@@ -130,7 +130,8 @@ typedef struct {
                                       half); the persistent kernel queues tile ids in the second half */
     uint32_t *sched;               /* 16 words: [0] active blocks, [1] next blocks, [2] done CTAs, [3] work items,
                                       [4] next items, [6..7] uint64 cells computed over real steps; the
-                                      persistent kernel's [10] step epoch, [11] start-list tiles taken and
+                                      persistent kernel's [8] epoch of the first idle step, [9] epoch of the last
+                                      step with a source outside the active blocks, [10] step epoch, [11] start-list tiles taken and
                                       [12..15] its two tile queues' lengths and taken counts; others zero */
     uint32_t *dt_buf;              /* 4 words per instance: [0] this step's dt (float bits, 0 = no-op),
                                       [1] the next step's CFL bound, [2..3] the persistent kernel's

@@ -36,6 +36,8 @@ constexpr int kSchedDone = 2;       // CTAs of the dilation that finished
 constexpr int kSchedItems = 3;      // tile work items of the current step
 constexpr int kSchedNextItems = 4;  // tile work items appended by the dilation
 constexpr int kSchedComputed = 6;   // [6,7]: uint64 cells computed over real steps
+constexpr int kSchedIdle = 8;       // epoch of the first step in which no instance runs (persistent kernel)
+constexpr int kSchedSrcOut = 9;     // epoch of the last step with a source in an inactive block (persistent kernel)
 constexpr int kSchedEpoch = 10;     // steps of the persistent kernel since the run's prologue
 constexpr int kSchedStartTaken = 11;  // tiles of the start list taken (persistent kernel)
 constexpr int kSchedQProd = 12;       // [12, 13]: tiles queued for steps of each parity (persistent kernel)
@@ -166,7 +168,8 @@ __device__ __forceinline__ uint32_t step_control(swe_ctrl_t *c, uint32_t *dt_buf
     const uint64_t now0 = c->now_ticks, stop = c->stop_ticks, steps0 = c->steps;
     const uint32_t done = c->dt_ticks, dt_max = c->dt_max_ticks, dry_dt = c->dry_dt_ticks;
     const float last0 = c->last_raw, safety = c->cfl_safety;
-    const uint32_t bound0 = dt_buf[0], bound1 = dt_buf[1];
+    const uint32_t bound0 = dt_buf[0];
+    const uint32_t bound1 = *reinterpret_cast<const volatile uint32_t *>(dt_buf + 1);  // minima may just have landed
     uint64_t now = now0, steps = steps0;
     float raw = last0;  // a no-op step computed no bound; RETARGET replans from the last one
     if (mode == 0) {

@@ -37,6 +37,15 @@ namespace swe {
 // arrive while it computes its fluxes); a dense step spreads the queue over all
 // CTAs.
 //
+// Sources: up to kFusedSources of them cost a step no barrier of their own. The CTA
+// that computes a tile adds its sources right after the tile's corrector (each thread
+// looks at a few of the listed cells, which stay in L1), and the CFL bounds, which need
+// every neighbour's depth after its own source, are taken by the step control's CTA.
+// A source in an inactive block (whose committed depth correctors of neighbouring
+// tiles read) waits for one more barrier, in the steps that have one: the step control
+// says so in advance. More sources than that (rain) run as two grid-wide passes with
+// a barrier before each.
+//
 // Step control: the last CTA to arrive at a step's final barrier runs it for
 // every instance after the others have gone on, and publishes each instance's
 // next dt beside that step's epoch as one 64-bit pair (dt words 2..3), which
@@ -52,6 +61,11 @@ namespace swe {
 // end of a launch one pass turns the last marks into the flags, block list and
 // tile work items the other kernels and the host read.
 constexpr uint32_t kExtraCap = 512;  // tiles a CTA computes besides its seat in one step
+// Sources up to which the fused form is taken: at most four list entries per thread and tile, read from L1.
+// 540 steps of a 30k-cell mesh with 7 inflows take 7.0 ms this way; with the two grid-wide passes (two more
+// barriers a step, one thread following a source's slots and marking its two-ring one block after the
+// other) they took 16.9 ms, 28 us a step.
+constexpr uint32_t kFusedSources = 1024;
 constexpr uint32_t kRingCache = 96;  // blocks of the seat's two-ring kept in shared memory
 constexpr uint32_t kNoTile = 0xFFFFFFFFu;
 
@@ -139,6 +153,40 @@ __device__ __forceinline__ void mark_ring_thread(const swe_mesh_t &m, const swe_
     }
 }
 
+// The sources of a tile's cells, right after its corrector (all threads; the tile's stores
+// are visible to the CTA): state0 != nullptr is the tile's committed state in shared
+// memory, columns h, hu, hv, h_lo. True for all threads when a source left a cell wet.
+__device__ __forceinline__ bool tile_sources(const swe_state_t &s, const swe_sources_t &src, const Phys &p, int comp,
+                                             const Item &it, float dt, float *state0) {
+    bool wet = false;
+    const uint32_t c0 = it.tile * kTileCells;
+    for (uint32_t k = threadIdx.x; k < src.count; k += blockDim.x) {
+        const uint32_t i = __ldg(src.cells + k);
+        if (i - c0 < it.cells)
+            wet |= source_add(s, src, k, i, it.inst, dt, p.dry_tol, comp, state0 ? state0 + (i - c0) : nullptr);
+    }
+    wet = __syncthreads_or(wet) != 0;
+    if (wet && threadIdx.x == 0) s.blk[kBlkWords * (it.tile >> 2) + kBlkWet] = 1u;
+    return wet;
+}
+
+// The sources of blocks that are not active in this step, one per warp of the grid in turn, after every
+// corrector: a source that wets its cell marks the block's two-ring.
+__device__ __forceinline__ void idle_block_sources(const swe_mesh_t &m, const swe_state_t &s, const swe_sources_t &src,
+                                                   const Phys &p, int comp, uint32_t epoch, uint32_t qpar) {
+    for (uint32_t k = blockIdx.x + gridDim.x * (threadIdx.x >> 5); k < src.count; k += gridDim.x * (blockDim.x >> 5)) {
+        const uint32_t i = __ldg(src.cells + k), b = i >> 8, inst = m.block_inst[b];
+        const uint32_t dt_bits = s.dt_buf[kDtWords * inst];
+        if (dt_bits == 0u || block_active(s.blk, b)) continue;
+        bool wet = false;
+        if ((threadIdx.x & 31u) == 0u) {
+            wet = source_add(s, src, k, i, inst, __uint_as_float(dt_bits), p.dry_tol, comp);
+            if (wet) s.blk[kBlkWords * b + kBlkWet] = 1u;
+        }
+        if (__any_sync(0xFFFFFFFFu, wet)) mark_ring(m, s, b, epoch, epoch + 1u, qpar, nullptr, 0u);
+    }
+}
+
 // Stage the tile of `item` into buffer k (warp 0): everything, or its state only.
 template <int STAGE>
 __device__ __forceinline__ void seat_issue(const swe_mesh_t &m, const swe_state_t &s, const uint4 item, const TileBuf &B,
@@ -218,7 +266,7 @@ __device__ __forceinline__ void seat_take(const swe_mesh_t &m, const swe_state_t
 template <bool COMP, bool CLAMP, bool OPEN>
 __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const Phys &p, float cfl,
                                unsigned char *smem, TiledShared<kPersistThreads> &sh, SeatShared &ss, uint32_t *ph,
-                               uint64_t &computed, uint32_t step, uint32_t epoch, bool all_active, bool sources) {
+                               uint64_t &computed, uint32_t step, uint32_t epoch, bool all_active, bool restage) {
     const TilePlan L = tile_plan(m.max_sub_edges, m.max_sub_slots, 10u);
     float *F = reinterpret_cast<float *>(smem + L.total);
     const TileBuf B0 = tile_buf(smem, L, 0u), B1 = tile_buf(smem, L, 1u);
@@ -231,7 +279,7 @@ __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const 
         // anyone reads). An open mesh's tallies need dt in the flux loop: no early start.
         const Item it = unpack(ss.seat_item);
         const uint32_t b = ss.seat >> 2;
-        if (!ss.state_ok || sources) {
+        if (!ss.state_ok || restage) {
             if (tid < 32u) seat_issue<0>(m, s, ss.seat_item, B0, true);
             if (!seat_wait(s, B0, ph, 0u)) return false;
         }
@@ -280,7 +328,7 @@ __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const 
     }
     __syncthreads();
     if (OPEN && ss.seat_active) {
-        if (!ss.state_ok || sources) {
+        if (!ss.state_ok || restage) {
             if (tid < 32u) seat_issue<0>(m, s, ss.seat_item, B0, true);
             if (!seat_wait(s, B0, ph, 0u)) return false;
         }
@@ -369,7 +417,7 @@ __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const 
         seat_take(m, s, ss, step, epoch, all_active);
         // every thread reads what decides its path before thread 0 changes it
         const uint32_t t = ss.take;
-        const bool seat_free = ss.seat == kNoTile, restage = ss.staged == t;
+        const bool seat_free = ss.seat == kNoTile, staged = ss.staged == t;
         __syncthreads();
         if (t == kNoTile) break;
         if (seat_free) {
@@ -382,8 +430,8 @@ __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const 
                 ss.staged = t;
                 ss.state_ok = 1u;
             }
-            if (tid < 32u) seat_issue<0>(m, s, ss.take_item, B0, restage);
-            if (!restage && tid >= 32u && tid < 64u) {
+            if (tid < 32u) seat_issue<0>(m, s, ss.take_item, B0, staged);
+            if (!staged && tid >= 32u && tid < 64u) {
                 // warp 1: the seat's two-ring and forced flag, while the records arrive
                 const uint32_t b = t >> 2, lane = tid & 31u;
                 const uint32_t k0 = m.ring_ptr[b], rn = m.ring_ptr[b + 1] - k0;
@@ -423,7 +471,8 @@ __device__ bool seat_predictor(const swe_mesh_t &m, const swe_state_t &s, const 
 template <bool COMP, bool CLAMP, bool OPEN>
 __device__ bool seat_corrector(const swe_mesh_t &m, const swe_state_t &s, const Phys &p, float cfl,
                                unsigned char *smem, TiledShared<kPersistThreads> &sh, SeatShared &ss, uint32_t *ph,
-                               uint64_t &computed, uint32_t step, uint32_t epoch, bool all_active) {
+                               uint64_t &computed, uint32_t step, uint32_t epoch, bool all_active,
+                               const swe_sources_t &src, bool fused) {
     const TilePlan L = tile_plan(m.max_sub_edges, m.max_sub_slots, 10u);
     float *F = reinterpret_cast<float *>(smem + L.total);
     const TileBuf B0 = tile_buf(smem, L, 0u), B1 = tile_buf(smem, L, 1u);
@@ -433,8 +482,9 @@ __device__ bool seat_corrector(const swe_mesh_t &m, const swe_state_t &s, const 
     if (n && tid < 32u) seat_issue<1>(m, s, ss.extra[0], B1, false);
     if (ss.seat_active) {
         const Item it = unpack(ss.seat_item);
-        const bool wet = tile_compute<1, COMP, CLAMP, kPersistThreads, OPEN>(
+        bool wet = tile_compute<1, COMP, CLAMP, kPersistThreads, OPEN>(
             m, s, p, cfl, B0, it, __uint_as_float(ss.seat_dt), 6u, 0u, F, L.capE, sh.red, computed, true);
+        if (fused) wet |= tile_sources(s, src, p, COMP ? 1 : 0, it, __uint_as_float(ss.seat_dt), B0.c);
         if (!all_active && tid < 32u && (wet || ss.seat_forced != 0u)) {
             const bool cached = ss.ring_n <= kRingCache;
             mark_ring(m, s, it.tile >> 2, epoch, next, qpar, cached ? ss.ring : nullptr, ss.ring_n,
@@ -447,8 +497,9 @@ __device__ bool seat_corrector(const swe_mesh_t &m, const swe_state_t &s, const 
         if (w > 0u && tid < 32u) seat_issue<1>(m, s, ss.extra[w], B1, false);
         if (!seat_wait(s, B1, ph, 1u)) return false;
         const Item it = unpack(ss.extra[w]);
-        const bool wet = tile_compute<1, COMP, CLAMP, kPersistThreads, OPEN>(
+        bool wet = tile_compute<1, COMP, CLAMP, kPersistThreads, OPEN>(
             m, s, p, cfl, B1, it, __uint_as_float(ss.extra_dt[w]), 0u, 6u, F, L.capE, sh.red, computed, false);
+        if (fused) wet |= tile_sources(s, src, p, COMP ? 1 : 0, it, __uint_as_float(ss.extra_dt[w]), nullptr);
         // the kept tile's block has its two-ring and this step's active bits cached
         const uint32_t eb = it.tile >> 2;
         const bool cached = ss.kept_ring_block == eb && ss.kept_bits_step == step + 1u && ss.kept_ring_n <= kRingCache;
@@ -538,6 +589,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
                 s.sched[kSchedQProd + k] = 0u;
                 s.sched[kSchedQCons + k] = 0u;
             }
+            s.sched[kSchedIdle] = s.sched[kSchedSrcOut] = 0u;  // no epoch of this launch
         }
     }
     if (blockIdx.x == 0)  // no published dt pair of an earlier run or launch carries an epoch of this one
@@ -549,19 +601,30 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
     auto nothing = [] {};
     uint32_t ph[2] = {0u, 0u};
     uint64_t computed = 0;
-    bool ok = true;
+    const bool fused = src.count != 0u && src.count <= kFusedSources;
+    bool ok = true, idle = false;
     uint32_t step = 0;
     for (; step < n_steps; ++step) {
         // E(n) = epoch0 + n + 1: never the zero the prologue leaves in the marks, never a value
         // of an earlier launch (each leaves its last E(n) + 1 in the epoch word)
         const uint32_t epoch = epoch0 + step + 1u, next_epoch = epoch + 1u;
         if (!(ok = seat_predictor<COMP, CLAMP, OPEN>(m, s, p, cfl, smem, sh, ss, ph, computed, step, epoch, all,
-                                                      src.count != 0u)))
+                                                      src.count != 0u && !fused)))
             break;
         if (!(ok = count_sync(g, flag, nothing))) break;
-        if (!(ok = seat_corrector<COMP, CLAMP, OPEN>(m, s, p, cfl, smem, sh, ss, ph, computed, step, epoch, all)))
+        // No instance runs this step (every window is done): the steps left do nothing either, 5 us each on a
+        // small mesh (8 fixed steps of 2048 cells took 1.02 ms of a 200-step launch). The last
+        // step's control wrote the word before its CTA came to the barrier just passed, so every CTA sees it.
+        if ((idle = *reinterpret_cast<volatile uint32_t *>(s.sched + kSchedIdle) == epoch)) break;
+        if (!(ok = seat_corrector<COMP, CLAMP, OPEN>(m, s, p, cfl, smem, sh, ss, ph, computed, step, epoch, all, src,
+                                                     fused)))
             break;
-        if (src.count) {
+        if (fused && !all &&
+            (step == 0u || *reinterpret_cast<volatile uint32_t *>(s.sched + kSchedSrcOut) == epoch)) {
+            if (!(ok = count_sync(g, flag, nothing))) break;
+            idle_block_sources(m, s, src, p, COMP ? 1 : 0, epoch, (step + 1u) & 1u);
+        }
+        if (src.count && !fused) {
             if (!(ok = count_sync(g, flag, nothing))) break;
             source_apply(m, s, src, p.dry_tol, COMP ? 1 : 0, first, stride);
             if (!(ok = count_sync(g, flag, nothing))) break;
@@ -576,19 +639,32 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         }
         const bool last_step = step + 1u == n_steps;
         auto control = [&] {
+            if (fused) {
+                source_bound_cta(m, s, src, p, cfl);
+                __syncthreads();  // the bounds land before step_control reads them
+            }
+            bool runs = false, out = false;
+            if (fused && !all)
+                for (uint32_t k = threadIdx.x; k < src.count; k += blockDim.x)
+                    out |= s.marks[2u * (__ldg(src.cells + k) >> 8)] != next_epoch;
+            out = __syncthreads_or(out) != 0;
             for (uint32_t i = threadIdx.x; i < m.n_inst; i += blockDim.x) {
                 const uint32_t dt = step_control(s.ctrl + i, s.dt_buf + kDtWords * i, 1);
+                runs |= dt != 0u;
                 // readers use the pair's own 64 bits only: no release ordering to wait for
                 st_relaxed_u64(const_cast<uint64_t *>(dt_pair(s, i)), (static_cast<uint64_t>(next_epoch) << 32) | dt);
             }
-            if (threadIdx.x == blockDim.x - 1u) {  // beside instance 0's control, not after it
+            const bool done = __syncthreads_or(runs) == 0;
+            if (threadIdx.x == blockDim.x - 1u) {
+                if (done) s.sched[kSchedIdle] = next_epoch;
+                if (out) s.sched[kSchedSrcOut] = next_epoch;
                 volatile uint32_t *sched = s.sched;
                 sched[kSchedEpoch] = next_epoch;
                 if (step == 0u) sched[kSchedStartTaken] = 0u;
                 // this step's queue is used up: it takes the tiles of the step after next
                 sched[kSchedQProd + (step & 1u)] = 0u;
                 sched[kSchedQCons + (step & 1u)] = 0u;
-                if (last_step) {  // the hand-over lists are counted from zero
+                if (last_step || done) {  // the hand-over lists are counted from zero
                     sched[kSchedActive] = 0u;
                     sched[kSchedItems] = 0u;
                     sched[kSchedNext] = 0u;
@@ -603,7 +679,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         // the hand-over reads the last step's dt and the lists its control zeroes
         if (last_step && !(ok = count_sync(g, flag, nothing))) break;
     }
-    if (ok && step > 0u) seat_handover(m, s, epoch0 + step + 1u, all);
+    if (ok && !idle && step > 0u) seat_handover(m, s, epoch0 + step + 1u, all);
     if (threadIdx.x == 0) {
         if (!ok) atomicOr(&s.ctrl->error, 2u);
         if (computed) atomicAdd(reinterpret_cast<unsigned long long *>(s.sched + kSchedComputed), computed);

@@ -34,6 +34,29 @@ __device__ __forceinline__ float clock_seconds(const swe_ctrl_t *c) {
     return static_cast<float>(c->now_ticks) * (1.0f / kTicksPerSecond);
 }
 
+// Source k's increment of cell i (of an instance whose step is dt), into the committed depth; keep != nullptr:
+// the cell's h also goes to keep[0] and its low word to keep[3 x 64] (a tile's state held in shared memory).
+// Returns whether the cell is wet after it.
+__device__ __forceinline__ bool source_add(const swe_state_t &s, const swe_sources_t &src, uint32_t k, uint32_t i,
+                                           uint32_t inst, float dt, float dry_tol, int comp, float *keep = nullptr) {
+    float rate = src.rate[k];
+    if (src.hydro && src.hydro[k] != 0xFFFFFFFFu)
+        rate = rate + src.hscale[k] * hydrograph_at(src, src.hydro[k], clock_seconds(s.ctrl + inst));
+    const float inc = dt * rate;
+    float h_new;
+    if (comp) {
+        float lo_new;
+        add_compensated(s.h[i], s.h_lo[i], inc, h_new, lo_new);
+        s.h_lo[i] = lo_new;
+        if (keep) keep[3 * kTileCells] = lo_new;
+    } else {
+        h_new = gmax(s.h[i] + inc, 0.0f);
+    }
+    s.h[i] = h_new;
+    if (keep) keep[0] = h_new;
+    return h_new >= dry_tol;
+}
+
 __device__ __forceinline__ void source_apply(const swe_mesh_t &m, const swe_state_t &s, const swe_sources_t &src,
                                              float dry_tol, int comp, uint32_t first, uint32_t stride) {
     for (uint32_t k = first; k < src.count; k += stride) {
@@ -41,21 +64,8 @@ __device__ __forceinline__ void source_apply(const swe_mesh_t &m, const swe_stat
         const uint32_t inst = m.block_inst[i >> 8];
         const uint32_t dt_bits = s.dt_buf[kDtWords * inst];
         if (dt_bits == 0u) continue;
-        const float dt = __uint_as_float(dt_bits);
-        float rate = src.rate[k];
-        if (src.hydro && src.hydro[k] != 0xFFFFFFFFu)
-            rate = rate + src.hscale[k] * hydrograph_at(src, src.hydro[k], clock_seconds(s.ctrl + inst));
-        const float inc = dt * rate;
-        float h_new;
-        if (comp) {
-            float lo_new;
-            add_compensated(s.h[i], s.h_lo[i], inc, h_new, lo_new);
-            s.h_lo[i] = lo_new;
-        } else {
-            h_new = gmax(s.h[i] + inc, 0.0f);
-        }
-        s.h[i] = h_new;
-        if (h_new >= dry_tol) s.blk[kBlkWords * (i >> 8) + kBlkWet] = 1u;
+        if (source_add(s, src, k, i, inst, __uint_as_float(dt_bits), dry_tol, comp))
+            s.blk[kBlkWords * (i >> 8) + kBlkWet] = 1u;
     }
 }
 
@@ -112,6 +122,57 @@ __device__ __forceinline__ void source_bound(const swe_mesh_t &m, const swe_stat
         acc = min(acc, b);
     }
     bound_flush_warp(s, acc_inst, acc);
+}
+
+// The post-source CFL bounds of a few sources by one CTA, eight lanes per source, one
+// CSR slot per lane: the slots' loads are in flight together, and the lanes' terms are
+// added in slot order, so the sums are source_bound's bit for bit. All threads.
+__device__ __forceinline__ void source_bound_cta(const swe_mesh_t &m, const swe_state_t &s, const swe_sources_t &src,
+                                                 const Phys &p, float cfl) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const uint32_t sub = threadIdx.x & 7u, groups = blockDim.x >> 3;
+    for (uint32_t k0 = 0; k0 < src.count; k0 += groups) {
+        const uint32_t k = k0 + (threadIdx.x >> 3);
+        bool run = k < src.count;
+        uint32_t i = 0u, inst = 0u, base = 0u, q = 0u, q1 = 0u;
+        float h = 0.0f, hu = 0.0f, hv = 0.0f, A = 0.0f;
+        if (run) {
+            i = __ldg(src.cells + k);
+            inst = m.block_inst[i >> 8];
+            base = m.tile_ptr[i >> 8];
+            q = m.cptr[i];
+            q1 = m.cptr[i + 1];
+            A = m.area[i];
+            h = s.h[i];
+            hu = s.hu[i];
+            hv = s.hv[i];
+            run = s.dt_buf[kDtWords * inst] != 0u && h >= p.dry_tol;
+        }
+        float u = 0.0f, c = 0.0f;
+        if (run) {
+            u = sqrtf(hu * hu + hv * hv) / h;
+            c = sqrtf(p.g * h);
+        }
+        float lam = 0.0f;
+        while (__any_sync(kFull, run && q < q1)) {
+            float term = 0.0f;
+            if (run && q + sub < q1) {
+                const uint32_t v = m.lcsr[q + sub];
+                const uint32_t e = base + (v >> 1);
+                const int nb = (v & 1u) ? m.tile_cl[e] : m.tile_cr[e];
+                const bool dry_side = nb >= 0 && s.h[nb] < p.dry_tol;
+                term = (u + (dry_side ? 2.0f : 1.0f) * c) * m.tile_len[e];
+            }
+            for (int l = 0; l < 8; ++l) {
+                const float t = __shfl_sync(kFull, term, l, 8);
+                if (q + l < q1) lam += t;
+            }
+            q += 8u;
+        }
+        uint32_t bound = kNoBound;
+        if (run && sub == 0u && lam > 1e-30f && A > 1e-10f) bound = __float_as_uint(cfl * A / lam);
+        bound_flush_warp(s, inst, bound);
+    }
 }
 
 }  // namespace swe
