@@ -287,8 +287,8 @@ def capture_chunks(solver, steps: int, chunk: int, timed: bool):
     from inundation_b200 import native
 
     graphs, events = [], []
-    if solver.stage_kernel == "persistent":
-        # one cooperative launch per chunk; its phases are not separate launches to time
+    if solver.stage_kernel in ("persistent", "staged"):
+        # one cooperative launch of whole steps per chunk; its phases are not separate launches to time
         left = steps
         while left > 0:
             n = min(chunk, left)
@@ -885,14 +885,14 @@ def run_sources_workload(args, world: int, rank: int, local: int, built=None) ->
     bpc = algorithmic_bytes_per_cell_step(g)
     peak, peak_kind = peaks()
     achieved = computed * bpc / (ms * 1e-3) / 1e9
-    stage_launches = 2 * args.steps if kernel != "persistent" else -(-args.steps // args.chunk)
+    whole = kernel in ("persistent", "staged")  # one cooperative launch of whole steps per chunk
+    stage_launches = 2 * args.steps if not whole else -(-args.steps // args.chunk)
     traffic = None
     tfile = ROOT / "profiles" / "stage_kernel_traffic.json"
     if tfile.exists():
         per_cell = json.loads(tfile.read_text()).get(kernel, {}).get("dram_bytes_per_computed_cell_step")
         if per_cell:
             traffic = per_cell * computed / stage_launches
-    per_step_launches = {"persistent": 0, "plain": 5, "staged": 5, "tiled": 5}[kernel]  # stages, sources (2), dilation
 
     # End to end through the public calls: the spun-up state from host arrays, a clock restart, the
     # same number of steps (the timed region's graphs, already captured), the final depth back.
@@ -928,7 +928,7 @@ def run_sources_workload(args, world: int, rank: int, local: int, built=None) ->
         "computed_cell_steps_per_s": world * computed / (ms_max * 1e-3),
         "active_fraction": computed / (g.N * args.steps),
         "simulated_s": t_sim,
-        "gpu_launches": per_step_launches * args.steps if kernel != "persistent" else stage_launches,
+        "gpu_launches": stage_launches if whole else 5 * args.steps,  # stages, sources (2), dilation
         "roofline": {
             "bound": "hbm",
             "achieved": achieved,
@@ -1053,7 +1053,9 @@ def run_batch(args, world: int, local: int) -> dict:
         raise RuntimeError("batched end-to-end run stalled")
     del finals
     kernel = solver.stage_kernel
-    launches_per_step = 3 + (2 if solver._src_count else 0)  # stages, dilation (+ source increments and bounds)
+    # stages, dilation (+ source increments and bounds), or one launch of whole steps for every 200
+    launches_per_step = 3 + (2 if solver._src_count else 0)
+    launches = -(-steps // 200) if kernel in ("persistent", "staged") else launches_per_step * steps
     del solver
     torch.cuda.empty_cache()
 
@@ -1104,7 +1106,7 @@ def run_batch(args, world: int, local: int) -> dict:
             "path": "BatchedSolver.reset(host states) + start + run_steps + download_h per scenario",
         },
         "build_s": t_build,
-        "gpu_launches": launches_per_step * steps,
+        "gpu_launches": launches,
         "clocks": clock,
     }
 

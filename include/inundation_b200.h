@@ -125,11 +125,12 @@ typedef struct {
     float *h1, *hu1, *hv1, *h1_lo; /* Heun predictor */
     float *clamp_mass;             /* per-cell positivity-clamp volume (diagnostic) */
     uint32_t *blk;                 /* 3 words per block: wet, active, forced */
-    uint32_t *active_list;         /* 2 x n_blocks: active blocks of the current step (first half) */
+    uint32_t *active_list;         /* 2 x n_blocks: active blocks of the current step (first half); the
+                                      second half is the listed blocks in the same order, then all others */
     uint32_t *items;               /* 2 x 4 words per 64-cell tile: work items of the tiled kernels (first
                                       half); the persistent kernel queues tile ids in the second half */
     uint32_t *sched;               /* 16 words: [0] active blocks, [1] next blocks, [2] done CTAs, [3] work items,
-                                      [4] next items, [6..7] uint64 cells computed over real steps; the
+                                      [4] next items, [5] unlisted blocks, [6..7] uint64 cells computed over real steps; the
                                       persistent kernel's [8] epoch of the first idle step, [9] epoch of the last
                                       step with a source outside the active blocks, [10] step epoch, [11] start-list tiles taken and
                                       [12..15] its two tile queues' lengths and taken counts; others zero */
@@ -189,6 +190,36 @@ typedef struct {
    persistent kernel that times out records error 2 in the control block. */
 int swe_steps(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
               const swe_sources_t *sources, uint32_t n_steps, swe_stream_t stream);
+
+/* The 256-cell tiles' records packed for swe_steps_blocks (device pointers), in the order of tile_*.
+   rec holds (nx, ny, len, cells) per record, 16-byte aligned, cells the bits of left | right << 16 as
+   indices into the block's cells: a cell of the block by its place in it, the k-th cell of the
+   block's halo list as 256 + k, 0xFFFF beyond a boundary edge. dz holds (dzl, dzr) per record. The
+   halo lists are halo[halo_ptr[b] .. halo_ptr[b + 1]): the cells outside block b that its records
+   name, each once; max_halo is the longest. perim is every cell's perimeter, the sum of its edges'
+   len, rounded up (at least 1e-5 above the sum). src_ptr: when a run has sources they come by
+   ascending cell, block b's being src_ptr[b] .. src_ptr[b + 1] - 1 (NULL without sources). */
+typedef struct {
+    const float *rec;
+    const float *dz;
+    const uint32_t *halo;
+    const uint32_t *halo_ptr; /* n_blocks + 1 */
+    const float *perim;       /* n_blocks * 256 */
+    const uint32_t *src_ptr;  /* n_blocks + 1 */
+    uint32_t max_halo;
+} swe_blocks_t;
+
+/* swe_steps for a mesh with many active blocks: n_steps whole steps, a 256-cell block at a time, in
+   one persistent cooperative launch from packed records (the mesh needs blk_lcsr too), and
+   a last launch that brings the flags, the block list and the work items up to date. The same
+   results. params->kernel is not read; params->grid caps the CTAs (0 = as many as fit). It uses the
+   barrier words and the dt pairs as kernel 2 does, and records the same errors. Not for a stream
+   being captured. */
+int swe_steps_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, const swe_state_t *state,
+                     const swe_params_t *params, const swe_sources_t *sources, uint32_t n_steps, swe_stream_t stream);
+
+/* CTAs per SM of swe_steps_blocks for this mesh; 0 when its largest block does not fit. */
+int swe_configure_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, int *blocks_per_sm);
 
 /* Bytes of device workspace of a mesh of n_blocks blocks and n_inst
    instances: active list, work items, sched words, dt words and control

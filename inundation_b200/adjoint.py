@@ -62,6 +62,7 @@ class GaugeCalibration(ResidentEngine):
     cut_depth: float = 0.0
     # the segment graphs capture one swe_step per step: a per-step stage kernel
     stage_kernel: str = "tiled"
+    packed_blocks: bool = False  # every step is one swe_step, and set_parameters moves the bed steps
     # reverse each segment in one cooperative launch (grid barriers between phases) instead of one
     # launch per phase and step; the arithmetic is the same. Off by default: at 250k cells the
     # per-phase launches fill more SMs and measured faster (121 against 135 ms for 2000 steps).

@@ -35,11 +35,13 @@ constexpr int kSchedNext = 1;       // blocks appended by the dilation
 constexpr int kSchedDone = 2;       // CTAs of the dilation that finished
 constexpr int kSchedItems = 3;      // tile work items of the current step
 constexpr int kSchedNextItems = 4;  // tile work items appended by the dilation
+constexpr int kSchedOthers = 5;     // unlisted blocks appended by the dilation
 constexpr int kSchedComputed = 6;   // [6,7]: uint64 cells computed over real steps
 constexpr int kSchedIdle = 8;       // epoch of the first step in which no instance runs (persistent kernel)
 constexpr int kSchedSrcOut = 9;     // epoch of the last step with a source in an inactive block (persistent kernel)
 constexpr int kSchedEpoch = 10;     // steps of the persistent kernel since the run's prologue
 constexpr int kSchedStartTaken = 11;  // tiles of the start list taken (persistent kernel)
+constexpr int kSchedTake = 12;        // blocks taken by the predictor's CTAs (dense kernel)
 constexpr int kSchedQProd = 12;       // [12, 13]: tiles queued for steps of each parity (persistent kernel)
 constexpr int kSchedQCons = 14;       // [14, 15]: tiles taken from those queues (persistent kernel)
 

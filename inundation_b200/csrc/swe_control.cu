@@ -22,7 +22,10 @@ namespace swe {
 // kDilateWarps warps appends its active blocks and tiles with one atomic each.
 // An instance on a no-op step (dt 0) keeps its flags and is left out of the
 // lists, unless force is set: its clock only moves again after a RETARGET,
-// which the host issues through a forced dilation.
+// which the host issues through a forced dilation. force 2 (the end of a whole-step
+// launch): the flags of every block, and the lists for the instances that go on.
+// The second half of the active list gets every block, the listed ones first and in
+// their order, the others after them: the order in which the dense kernel's CTAs take blocks.
 // ---------------------------------------------------------------------------
 constexpr int kDilateWarps = 32;
 
@@ -35,8 +38,8 @@ __global__ void __launch_bounds__(kDilateWarps * 32)
     uint32_t v = 0u;
     if (b < m.n_blocks) {
         const uint32_t inst = m.block_inst[b];
-        const bool run = force || s.dt_buf[kDtWords * inst] != 0u;
-        if (run) {
+        const bool goes_on = s.dt_buf[kDtWords * inst] != 0u;
+        if (force || goes_on) {
             if (all_active) {
                 v = 1u;
             } else {
@@ -49,6 +52,7 @@ __global__ void __launch_bounds__(kDilateWarps * 32)
                 v = __any_sync(0xFFFFFFFFu, v != 0u) ? 1u : 0u;
             }
             if (lane == 0) s.blk[kBlkWords * b + kBlkActive] = v;
+            if (force == 2 && !goes_on) v = 0u;
         }
     }
     if (lane == 0) flag[warp] = v;
@@ -66,16 +70,23 @@ __global__ void __launch_bounds__(kDilateWarps * 32)
         }
         const uint32_t items_total = __shfl_sync(0xFFFFFFFFu, items_before, 31);
         items_before -= n_items;
-        uint32_t pos = 0, ipos = 0;
+        const unsigned others = __ballot_sync(0xFFFFFFFFu, !on && blk < m.n_blocks);
+        uint32_t pos = 0, ipos = 0, opos = 0;
         if (lane == 0 && ballot) {
             pos = atomicAdd(&s.sched[kSchedNext], static_cast<uint32_t>(__popc(ballot)));
             ipos = atomicAdd(&s.sched[kSchedNextItems], items_total);
+        }
+        if (lane == 1 && others) opos = atomicAdd(&s.sched[kSchedOthers], static_cast<uint32_t>(__popc(others)));
+        opos = __shfl_sync(0xFFFFFFFFu, opos, 1);
+        if ((others >> lane) & 1u) {
+            const uint32_t at = opos + __popc(others & ((1u << lane) - 1u));
+            if (at < m.n_blocks) s.active_list[2u * m.n_blocks - 1u - at] = blk;
         }
         pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
         ipos = __shfl_sync(0xFFFFFFFFu, ipos, 0) + items_before;
         if (on) {
             const uint32_t slot = pos + __popc(ballot & ((1u << lane) - 1u));
-            if (slot < m.n_blocks) s.active_list[slot] = blk;
+            if (slot < m.n_blocks) s.active_list[slot] = s.active_list[m.n_blocks + slot] = blk;
             const uint32_t inst = m.block_inst[blk];
             uint4 *out = reinterpret_cast<uint4 *>(s.items);
             for (uint32_t q = 0; q < n_items && ipos + q < 4u * m.n_blocks; ++q) {
@@ -102,6 +113,7 @@ __global__ void __launch_bounds__(kDilateWarps * 32)
         sched[kSchedItems] = sched[kSchedNextItems];
         sched[kSchedNext] = 0u;
         sched[kSchedNextItems] = 0u;
+        sched[kSchedOthers] = 0u;
         sched[kSchedDone] = 0u;
     }
 }
@@ -188,6 +200,13 @@ __global__ void source_apply_kernel(swe_mesh_t m, swe_state_t s, swe_sources_t s
 
 __global__ void source_bound_kernel(swe_mesh_t m, swe_state_t s, swe_sources_t src, Phys p, float cfl) {
     source_bound(m, s, src, p, cfl, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// Flags, block list and work items after a whole-step launch whose blocks kept their own flags.
+int launch_handover(const swe_mesh_t *m, const swe_state_t *s, const swe_params_t *p, cudaStream_t st) {
+    dilate_compact_kernel<<<(m->n_blocks + kDilateWarps - 1) / kDilateWarps, kDilateWarps * 32, 0, st>>>(
+        *m, *s, p->active_set ? 0 : 1, 2, -1);
+    return check_launch();
 }
 
 inline size_t cfl_smem_bytes(uint32_t max_tile_edges) { return ((max_tile_edges + 3u) & ~3u) * sizeof(float); }

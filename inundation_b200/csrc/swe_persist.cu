@@ -61,11 +61,6 @@ namespace swe {
 // end of a launch one pass turns the last marks into the flags, block list and
 // tile work items the other kernels and the host read.
 constexpr uint32_t kExtraCap = 512;  // tiles a CTA computes besides its seat in one step
-// Sources up to which the fused form is taken: at most four list entries per thread and tile, read from L1.
-// 540 steps of a 30k-cell mesh with 7 inflows take 7.0 ms this way; with the two grid-wide passes (two more
-// barriers a step, one thread following a source's slots and marking its two-ring one block after the
-// other) they took 16.9 ms, 28 us a step.
-constexpr uint32_t kFusedSources = 1024;
 constexpr uint32_t kRingCache = 96;  // blocks of the seat's two-ring kept in shared memory
 constexpr uint32_t kNoTile = 0xFFFFFFFFu;
 
@@ -540,6 +535,14 @@ __device__ __forceinline__ void seat_handover(const swe_mesh_t &m, const swe_sta
             s.blk[kBlkWords * b + kBlkActive] = listed ? 1u : 0u;
         }
         const uint32_t mask = __ballot_sync(0xFFFFFFFFu, listed);
+        const uint32_t others = __ballot_sync(0xFFFFFFFFu, !listed && b < m.n_blocks);
+        if (others) {  // the second half of the list: the listed blocks, then the others
+            uint32_t opos = 0u;
+            if (lane == 0) opos = atomicAdd(&s.sched[kSchedQCons], __popc(others));
+            opos = __shfl_sync(0xFFFFFFFFu, opos, 0);
+            if ((others >> lane) & 1u)
+                s.active_list[2u * m.n_blocks - 1u - (opos + __popc(others & ((1u << lane) - 1u)))] = b;
+        }
         if (!mask) continue;
         const uint32_t cells = listed ? m.block_cells[b] : 0u;
         const uint32_t n_items = (cells + kTileCells - 1u) / kTileCells;
@@ -558,7 +561,8 @@ __device__ __forceinline__ void seat_handover(const swe_mesh_t &m, const swe_sta
         pos0 = __shfl_sync(0xFFFFFFFFu, pos0, 0);
         ipos0 = __shfl_sync(0xFFFFFFFFu, ipos0, 0);
         if (listed) {
-            s.active_list[pos0 + __popc(mask & ((1u << lane) - 1u))] = b;
+            const uint32_t slot = pos0 + __popc(mask & ((1u << lane) - 1u));
+            s.active_list[slot] = s.active_list[m.n_blocks + slot] = b;
             uint4 *items = reinterpret_cast<uint4 *>(s.items);
             const uint32_t inst = m.block_inst[b];
             for (uint32_t q = 0; q < n_items; ++q) items[ipos0 + before + q] = tile_item(m, 4u * b + q, inst);
@@ -669,6 +673,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
                     sched[kSchedItems] = 0u;
                     sched[kSchedNext] = 0u;
                     sched[kSchedNextItems] = 0u;
+                    sched[kSchedQCons] = 0u;  // no queue is taken from any more: counts the unlisted blocks
                     sched[kSchedStartTaken] = 0u;
                 }
             }

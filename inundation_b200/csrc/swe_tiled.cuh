@@ -172,12 +172,16 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// safe_vel2 of both sides: the velocities of momenta q1, q2 at depth h, per lane.
-__device__ __forceinline__ void safe_vel_pair(const Phys &p, float2 h, float2 q1, float2 q2, float2 &v1, float2 &v2) {
+// The reciprocal of safe_vel2's denominator at depth h.
+__device__ __forceinline__ float vel_inv(const Phys &p, float h) {
     const float e = kFilmDepths * p.dry_tol;
-    const float2 hh = mul2(h, h);
-    const float2 den = add2(hh, pr(gmax(hh.x, e * e), gmax(hh.y, e * e)));
-    const float2 inv = pr(1.0f / den.x, 1.0f / den.y);
+    const float hh = h * h;
+    return 1.0f / (hh + gmax(hh, e * e));
+}
+
+// safe_vel2 of both sides: the velocities of momenta q1, q2 at depth h, per lane, from inv = vel_inv(h).
+__device__ __forceinline__ void safe_vel_pair(const Phys &p, float2 h, float2 inv, float2 q1, float2 q2, float2 &v1,
+                                              float2 &v2) {
     const float2 twice = mul2(pr(2.0f, 2.0f), h);
     v1 = mul2(mul2(twice, q1), inv);
     v2 = mul2(mul2(twice, q2), inv);
@@ -185,19 +189,24 @@ __device__ __forceinline__ void safe_vel_pair(const Phys &p, float2 h, float2 q1
     if (!(h.y > p.dry_tol)) v1.y = v2.y = 0.0f;
 }
 
-// face_states + hllc: the reconstructed depths hs and the face-frame HLLC flux and speed bound.
-__device__ __forceinline__ void face_flux_pair(const Phys &p, float nx, float ny, float2 dz, float2 h, float2 hu,
-                                               float2 hv, float2 &hs, float &Fh, float &Fhn, float &Fht,
-                                               float &smax) {
+// face_states + hllc from the cells' velocities u, v and inv = vel_inv(h): the reconstructed depths hs and
+// the face-frame HLLC flux and speed bound. The face sits on the higher of two beds, so one side's depth
+// is the cell's own (its step is zero) and vel_inv(hs) there is the value at hand: one reciprocal per edge
+// for the other side instead of two.
+__device__ __forceinline__ void face_flux_from_vel(const Phys &p, float nx, float ny, float2 dz, float2 h, float2 u,
+                                                   float2 v, float2 inv, float2 &hs, float &Fh, float &Fhn, float &Fht,
+                                                   float &smax) {
     const float2 dh = add2(h, pr(-dz.x, -dz.y));
     hs = pr(gmax(0.0f, dh.x), gmax(0.0f, dh.y));
-    float2 u, v;
-    safe_vel_pair(p, h, hu, hv, u, v);
     const float2 hus = mul2(hs, u), hvs = mul2(hs, v);
     const float2 qn = fma2(hus, pr(nx, nx), mul2(hvs, pr(ny, ny)));
     const float2 qt = fma2(hvs, pr(nx, nx), mul2(hus, pr(-ny, -ny)));
+    const bool ownL = hs.x == h.x, ownR = hs.y == h.y;
+    const float other = vel_inv(p, ownL ? hs.y : hs.x);
+    float2 invs = pr(ownL ? inv.x : other, ownR ? inv.y : other);
+    if (!ownL && !ownR) invs.y = vel_inv(p, hs.y);  // beds and steps that do not match: both depths differ
     float2 un, ut;
-    safe_vel_pair(p, hs, qn, qt, un, ut);
+    safe_vel_pair(p, hs, invs, qn, qt, un, ut);
     const float sqL = sqrtf(gmax(hs.x, 0.0f)), sqR = sqrtf(gmax(hs.y, 0.0f));
     const float root_g = sqrtf(p.g);
     const float2 c = mul2(pr(root_g, root_g), pr(sqL, sqR));
@@ -236,6 +245,33 @@ __device__ __forceinline__ void face_flux_pair(const Phys &p, float nx, float ny
     }
 }
 
+// The same from the cells' momenta.
+__device__ __forceinline__ void face_flux_pair(const Phys &p, float nx, float ny, float2 dz, float2 h, float2 hu,
+                                               float2 hv, float2 &hs, float &Fh, float &Fhn, float &Fht,
+                                               float &smax) {
+    const float2 inv = pr(vel_inv(p, h.x), vel_inv(p, h.y));
+    float2 u, v;
+    safe_vel_pair(p, h, inv, hu, hv, u, v);
+    face_flux_from_vel(p, nx, ny, dz, h, u, v, inv, hs, Fh, Fhn, Fht, smax);
+}
+
+// The gather words of a flux: its mass Fh and momentum Fhn, Fht in the face frame, with the hydrostatic terms.
+__device__ __forceinline__ void flux_words(const Phys &p, float nx, float ny, float len, float2 h, float2 hs, float Fh,
+                                           float Fhn, float Fht, float smax, float &w0, float &w1, float &w2,
+                                           float &w3, float &w4, float &w5) {
+    const float2 F = fma2(pr(Fhn, Fhn), pr(nx, ny), mul2(pr(Fht, Fht), pr(-ny, nx)));
+    const float2 hs2 = mul2(hs, hs);
+    const float2 hyd = mul2(pr(0.5f * p.g, 0.5f * p.g), fma2(h, h, pr(-hs2.x, -hs2.y)));
+    const float2 wn = mul2(fma2(hyd, pr(nx, nx), pr(F.x, F.x)), pr(len, len));
+    const float2 wt = mul2(fma2(hyd, pr(ny, ny), pr(F.y, F.y)), pr(len, len));
+    w0 = Fh * len;
+    w1 = wn.x;
+    w2 = wt.x;
+    w3 = wn.y;
+    w4 = wt.y;
+    w5 = smax * len;
+}
+
 // Flux of one edge from its two cell states: the five gather words and the
 // corrector's CFL word (resident.py:254-284). On an open edge (cR < -1,
 // condition kind/value) the mass flux follows the condition, and an
@@ -260,18 +296,9 @@ __device__ __forceinline__ void edge_words(const Phys &p, int cR, float nx, floa
     } else if (cR < 0) {
         Fh = 0.0f;  // a wall passes no mass
     }
-    const float2 F = fma2(pr(Fhn, Fhn), pr(nx, ny), mul2(pr(Fht, Fht), pr(-ny, nx)));
-    const float2 hs2 = mul2(hs, hs);
-    const float2 hyd = mul2(pr(0.5f * p.g, 0.5f * p.g), fma2(pr(hL, hR), pr(hL, hR), pr(-hs2.x, -hs2.y)));
-    const float2 wn = mul2(fma2(hyd, pr(nx, nx), pr(F.x, F.x)), pr(len, len));
-    const float2 wt = mul2(fma2(hyd, pr(ny, ny), pr(F.y, F.y)), pr(len, len));
-    w0 = Fh * len;
-    w1 = wn.x;
-    w2 = wt.x;
-    w3 = wn.y;
-    w4 = wt.y;
-    w5 = smax * len;
+    flux_words(p, nx, ny, len, pr(hL, hR), hs, Fh, Fhn, Fht, smax, w0, w1, w2, w3, w4, w5);
 }
+
 // ---------------------------------------------------------------------------
 // 64-cell tiles from work items, staged by bulk copies.
 // ---------------------------------------------------------------------------

@@ -22,7 +22,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import native
-from .layout import TileLayout
+from .layout import TileLayout, TileSet
 from .sources import NO_HYDROGRAPH, Hydrograph
 from .tuning import ACTIVE_BLOCK_CELLS, B200_BACKEND, CFL_DEFAULT, DRY_TOL_DEFAULT, GRAVITY_G, OPEN_INFLOW, OPEN_STAGE
 
@@ -50,6 +50,8 @@ KERNELS = {"tiled": 0, "plain": 1, "persistent": 2, "staged": 3}
 # whole GPU), unless every active tile still has a CTA of the persistent grid to itself (a small mesh).
 AUTO_DENSE_FRACTION = 0.25
 PERSISTENT_EXTRA_TILES = 512  # kExtraCap of the persistent kernel
+
+DENSE_TAKEN_BLOCKS = 512  # kTakenCap of the dense whole-step kernel
 
 
 def _i32(a: NDArray) -> NDArray[np.int32]:
@@ -84,11 +86,13 @@ class ResidentEngine:
     track_clamp: bool = False
     cfl_safety: float = 1.0
     # Stage kernel: "tiled" (64-cell tiles from the dilation's work items, staged by bulk copies),
-    # "plain" (256-cell blocks, direct loads), "staged" (256-cell blocks staged by bulk copies),
-    # "persistent" (the tiled stages and the rest of the
-    # step in one cooperative launch per submit, phases separated by grid barriers) or "auto"
+    # "plain" (256-cell blocks, direct loads), "staged" (256-cell blocks from packed records) and
+    # "persistent" (the tiled stages): the last two run whole steps in one cooperative launch per
+    # submit, phases separated by grid barriers; or "auto"
     # (persistent or staged by the active fraction read after every submit). All give the same bits.
     stage_kernel: str = "auto"
+    # keep the packed records with which the staged kernel runs whole steps (else it runs stage by stage)
+    packed_blocks: bool = True
 
     def _init_engine(
         self,
@@ -165,8 +169,37 @@ class ResidentEngine:
             self._per_sm[kernel] = max(1, per_sm.value)
             if kernel == KERNELS["staged"]:  # 0: the mesh's largest block does not fit its shared memory
                 self._staged_fits = per_sm.value > 0
+        self._pack_blocks(t, B)
         self.ctas_per_sm: int | None = None  # None: as many as fit
         self.max_grid: int | None = None  # an upper bound on the persistent CTAs (None: none)
+
+    def _pack_blocks(self, t: dict[str, torch.Tensor], B: TileSet) -> None:
+        """The 256-cell tiles' records as the dense whole-step kernel reads them, packed on the device from the
+        uploaded arrays: (nx, ny, len, local cells) and (dzl, dzr) side by side."""
+        self._blocks = None
+        if not self._staged_fits or not self.packed_blocks:
+            return
+        local = self._dev(_i32(B.local)).view(torch.float32)
+        self._blocks_t = {
+            "rec": torch.stack([t["tile_nx"], t["tile_ny"], t["tile_len"], local], dim=1),
+            "dz": torch.stack([t["tile_dzl"], t["tile_dzr"]], dim=1),
+            "halo": self._dev(B.halo), "halo_ptr": self._dev(_i32(B.halo_ptr)),
+        }
+        # every cell's perimeter, rounded up by more than the order of summing its edges can change
+        own = (local.view(torch.int32) & 0xFFFF) < B.tile_cells  # records in the tile of their left cell: each edge once
+        inner = own & (t["tile_cr"] >= 0)
+        around = torch.zeros(self.layout.n_padded_cells, dtype=torch.float64, device=self.device)
+        length = t["tile_len"].double()
+        around.index_add_(0, t["tile_cl"], torch.where(own, length, 0.0))
+        around.index_add_(0, t["tile_cr"].clamp(min=0), torch.where(inner, length, 0.0))
+        self._blocks_t["perim"] = (around * (1.0 + 1e-4)).float()
+        blocks = native.SweBlocks(max_halo=B.max_halo, **{k: v.data_ptr() for k, v in self._blocks_t.items()})
+        per_sm = ctypes.c_int(0)
+        with torch.cuda.device(self.device):
+            native.check(self._lib.swe_configure_blocks(ctypes.byref(self._mesh), ctypes.byref(blocks),
+                                                        ctypes.byref(per_sm)), "swe_configure_blocks")
+        if per_sm.value > 0:
+            self._blocks, self._dense_per_sm = blocks, per_sm.value
 
     def grid(self, kernel: int | None = None) -> int:
         """Persistent CTAs of a stage kernel: CTAs per SM x SMs, at most one per work unit."""
@@ -312,6 +345,10 @@ class ResidentEngine:
         self._src_count = int(cells.size)
         self._src_cells = dev(cells.astype(np.int32) if cells.size else np.zeros(1, np.int32))
         self._src_rate = dev(rate.astype(np.float32) if cells.size else np.zeros(1, np.float32))
+        if self._blocks is not None:  # the sources of every block, by ascending cell
+            bounds = np.arange(self.n_blocks + 1) * ACTIVE_BLOCK_CELLS
+            self._src_ptr = dev(np.searchsorted(host[0], bounds).astype(np.int32)) if self._src_count else None
+            self._blocks.src_ptr = self._src_ptr.data_ptr() if self._src_count else None
         self._src_hydro = None
         if hidx is not None and knots:
             ptr = np.zeros(len(knots) + 1, np.int64)
@@ -490,10 +527,14 @@ class ResidentEngine:
         native.check(self._lib.swe_steps(mesh, state, pp, sp, n_steps, stream), "swe_steps")
 
     def _graph(self, steps: int | None = None):
-        """A replayable submit of ``steps`` steps: a CUDA graph, or for the persistent kernel its one launch."""
+        """A replayable submit of ``steps`` steps: one whole-step launch (persistent, staged) or a CUDA graph of them."""
         steps = self.steps_per_graph if steps is None else steps
         if self._kernel == KERNELS["persistent"]:
             return _PersistentSubmit(self, steps)
+        if self._kernel == KERNELS["staged"] and self._blocks is not None:
+            submit = _DenseSubmit(self, steps)
+            if submit.fits:
+                return submit
         key = (
             steps,
             bool(self.compensated),
@@ -532,7 +573,7 @@ def _same_sources(a: list, b: list) -> bool:
 
 
 class _PersistentSubmit:
-    """One cooperative launch of the persistent kernel per replay (its own grid barriers replace the graph)."""
+    """One cooperative launch of whole steps per replay (its own grid barriers replace the graph)."""
 
     def __init__(self, engine: ResidentEngine, steps: int) -> None:
         self.engine, self.steps = engine, steps
@@ -544,6 +585,27 @@ class _PersistentSubmit:
             e._lib.swe_steps(ctypes.byref(e._mesh), ctypes.byref(e._state), ctypes.byref(self.params),
                              ctypes.byref(self.sources), self.steps, e._cuda_stream),
             "swe_steps",
+        )
+
+
+class _DenseSubmit(_PersistentSubmit):
+    """The same with the dense whole-step kernel on packed 256-cell blocks."""
+
+    def __init__(self, engine: ResidentEngine, steps: int) -> None:
+        super().__init__(engine, steps)
+        self.blocks = native.SweBlocks.from_buffer_copy(engine._blocks)  # with the sources of now
+        per_sm = engine._dense_per_sm if engine.ctas_per_sm is None else min(engine.ctas_per_sm, engine._dense_per_sm)
+        grid = min(engine.n_blocks, per_sm * engine._sms)
+        self.params.grid = max(1, grid if engine.max_grid is None else min(grid, engine.max_grid))
+        # every block of a step finds a CTA with room for it
+        self.fits = engine.n_blocks <= self.params.grid * DENSE_TAKEN_BLOCKS
+
+    def replay(self) -> None:
+        e = self.engine
+        native.check(
+            e._lib.swe_steps_blocks(ctypes.byref(e._mesh), ctypes.byref(self.blocks), ctypes.byref(e._state),
+                                    ctypes.byref(self.params), ctypes.byref(self.sources), self.steps, e._cuda_stream),
+            "swe_steps_blocks",
         )
 
 

@@ -43,6 +43,7 @@ from .tuning import ACTIVE_BLOCK_CELLS, num_blocks
 TILE_ALIGN = 32
 SUB_TILE_CELLS = 64
 MAX_TILE_EDGES = 32767
+NO_CELL = 0xFFFF  # local index beyond a boundary edge
 
 
 @dataclass
@@ -66,6 +67,16 @@ class TileSet:
     lcsr: NDArray[np.uint16]  # per CSR slot, flat in global slot order
     lcsr_blk: NDArray[np.uint16]  # the same, regrouped per tile from lcsr_ptr[t]
     lcsr_ptr: NDArray[np.uint32]  # n_tiles + 1, multiples of 8 (16-byte aligned segments)
+    # The cells a tile's records read outside it, each once, by cell id, and every record's two cells as
+    # tile-local indices, left | right << 16: a cell of the tile by its place in it, the k-th halo cell as
+    # tile_cells + k, NO_CELL beyond a boundary edge.
+    halo: NDArray[np.int32] | None = None
+    halo_ptr: NDArray[np.uint32] | None = None  # n_tiles + 1
+    local: NDArray[np.uint32] | None = None
+
+    @property
+    def max_halo(self) -> int:
+        return 0 if self.halo_ptr is None else int(np.diff(self.halo_ptr.astype(np.int64)).max())
 
 
 @dataclass
@@ -190,6 +201,33 @@ def _tile_set(geom: MeshGeometry, order: NDArray[np.int64], signed: NDArray[np.i
     )
 
 
+def _add_halo(T: TileSet, n_cells: int) -> None:
+    """The halo lists and local record indices of a tile set (see ``TileSet``)."""
+    size = T.tile_cells
+    tile = np.repeat(np.arange(T.n_tiles, dtype=np.int64), np.diff(T.ptr.astype(np.int64)))
+    base = tile * size
+    cl, cr = T.cl.astype(np.int64), T.cr.astype(np.int64)
+    real = T.edge >= 0
+    out_l = real & ((cl < base) | (cl >= base + size))
+    out_r = real & (cr >= 0) & ((cr < base) | (cr >= base + size))
+    at_l, at_r = np.flatnonzero(out_l), np.flatnonzero(out_r)
+    key = np.concatenate([tile[at_l] * n_cells + cl[at_l], tile[at_r] * n_cells + cr[at_r]])
+    unique, place = np.unique(key, return_inverse=True)
+    owner = unique // n_cells
+    ptr = np.searchsorted(owner, np.arange(T.n_tiles + 1))
+    T.halo = (unique - owner * n_cells).astype(np.int32) if unique.size else np.zeros(1, np.int32)
+    T.halo_ptr = ptr.astype(np.uint32)
+    if size + T.max_halo >= NO_CELL:
+        raise ValueError(f"a tile reads {T.max_halo} cells outside it; the limit is {NO_CELL - size - 1}")
+    slot = size + place - ptr[owner[place]]
+    left, right = cl - base, cr - base
+    left[at_l] = slot[: at_l.size]
+    right[at_r] = slot[at_l.size :]
+    right[cr < 0] = NO_CELL
+    left[~real] = right[~real] = 0
+    T.local = (left | (right << 16)).astype(np.uint32)
+
+
 def build_tile_layout(geom: MeshGeometry) -> TileLayout:
     """Both tile sets, the padded CSR pointers and the block two-ring of a Hilbert-ordered geometry."""
     n = int(geom.N)
@@ -220,12 +258,14 @@ def _build(geom) -> TileLayout:
     ecl = geom.edge_cellL[order].astype(np.int32)
     ecr = geom.edge_cellR[order].astype(np.int32)
     rptr, ridx = block_two_ring(*block_adjacency(ecl, ecr, n, bc))
+    blocks = _tile_set(geom, order, signed, bc)
+    _add_halo(blocks, n)
     return TileLayout(
         n_cells=n,
         n_edges=n_e,
         n_blocks=n_blk,
         edge_order=order,
-        blocks=_tile_set(geom, order, signed, bc),
+        blocks=blocks,
         subs=_tile_set(geom, order, signed, SUB_TILE_CELLS),
         cptr=cptr_pad.astype(np.uint32),
         ring_ptr=rptr.astype(np.uint32),

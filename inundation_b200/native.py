@@ -35,6 +35,8 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "swe_prologue": ([_P, _P, _P, _P], ctypes.c_int),
     "swe_step": ([_P, _P, _P, _P, _P], ctypes.c_int),
     "swe_steps": ([_P, _P, _P, _P, _U32, _P], ctypes.c_int),
+    "swe_steps_blocks": ([_P, _P, _P, _P, _P, _U32, _P], ctypes.c_int),
+    "swe_configure_blocks": ([_P, _P, ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
     "swe_volume_partials": ([_U32], _U32),
     "swe_volume_fp64": ([_P, _P, _P, _U32, _P, _P, _P], ctypes.c_int),
     "swe_volume_fp64_noalloc": ([_P, _P, _P, _U32, _P, _P], ctypes.c_int),
@@ -73,6 +75,10 @@ class SweMesh(ctypes.Structure):
         ("blk_lcsr", _P),
         ("blk_lcsr_ptr", _P),
     ]
+
+
+class SweBlocks(ctypes.Structure):
+    _fields_ = [*[(name, _P) for name in ("rec", "dz", "halo", "halo_ptr", "perim", "src_ptr")], ("max_halo", _U32)]
 
 
 class SweState(ctypes.Structure):
