@@ -195,10 +195,12 @@ int swe_steps(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params
    rec holds (nx, ny, len, cells) per record, 16-byte aligned, cells the bits of left | right << 16 as
    indices into the block's cells: a cell of the block by its place in it, the k-th cell of the
    block's halo list as 256 + k, 0xFFFF beyond a boundary edge. dz holds (dzl, dzr) per record. The
-   halo lists are halo[halo_ptr[b] .. halo_ptr[b + 1]): the cells outside block b that its records
-   name, each once; max_halo is the longest. perim is every cell's perimeter, the sum of its edges'
-   len, rounded up (at least 1e-5 above the sum). src_ptr: when a run has sources they come by
-   ascending cell, block b's being src_ptr[b] .. src_ptr[b + 1] - 1 (NULL without sources). */
+   steps lie in [0, 2^19] and the normals are unit vectors (what the branch-free operations' range
+   check relies on). The halo lists are halo[halo_ptr[b] .. halo_ptr[b + 1]): the cells outside block
+   b that its records name, each once; max_halo is the longest. perim is every cell's perimeter, the
+   sum of its edges' len, rounded up (at least 1e-5 above the sum). src_ptr: when a run has sources
+   they come by ascending cell, block b's being src_ptr[b] .. src_ptr[b + 1] - 1 (NULL without
+   sources). */
 typedef struct {
     const float *rec;
     const float *dz;
@@ -401,6 +403,11 @@ int swe_dt_wait_probe(const swe_state_t *state, uint32_t epoch, uint32_t *out, s
    (Sf = g n^2 |u| h^(-4/3)) as the update evaluates it. Replaces the pow(h, 4/3) of
    update_resident_gather (resident.py:489-495), for tests of its accuracy. */
 int swe_inv_pow43(const float *x, float *out, uint32_t n, swe_stream_t stream);
+
+/* The flux's branch-free operations on n pairs, on the device: out[0..n) = 1 / b, out[n..2n) = a / b and
+   out[2n..3n) = sqrt(b), each equal to the IEEE operation for a and b as the flux uses them (b positive, both
+   between 2^-80 and 2^62, a also negative or zero). For tests: no counterpart in the reference. */
+int swe_plain_math_probe(const float *a, const float *b, float *out, uint32_t n, swe_stream_t stream);
 
 const char *swe_status_string(int status);
 

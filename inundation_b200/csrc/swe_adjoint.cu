@@ -178,7 +178,7 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
     safe_vel2(p, hRs, hqnR, hqtR, unR, utR);
     const float sqL = sqrtf(gmax(hLs, 0.0f));
     const float sqR = sqrtf(gmax(hRs, 0.0f));
-    const float root_g = sqrtf(p.g);
+    const float root_g = p.root_g;
     const float cL = root_g * sqL;
     const float cR = root_g * sqR;
     const float den = sqL + sqR;
@@ -749,7 +749,7 @@ int swe_adjoint_segment(const swe_mesh_t *mesh, const swe_params_t *params, cons
     int rc = set_smem(adj_edge_kernel<0>, bytes);
     if (!rc) rc = set_smem(adj_edge_kernel<1>, bytes);
     if (rc) return rc;
-    const Phys ph{params->g, params->dry_tol};
+    const Phys ph = make_phys(params->g, params->dry_tol);
     const uint32_t n = mesh->n_blocks * kBlockCells;
     if (adj->sync) {
         auto kern = adj_persistent_kernel;
@@ -767,7 +767,7 @@ int swe_adjoint_segment(const swe_mesh_t *mesh, const swe_params_t *params, cons
         swe_adjoint_t aa = *adj;
         swe_sources_t sc = *sources;
         swe_gauges_t gg = *gauges;
-        Phys ph{params->g, params->dry_tol};
+        Phys ph = make_phys(params->g, params->dry_tol);
         uint32_t sl = slots, r0 = row0, t0 = tag0;
         void *args[] = {&mm, &tt, &aa, &sc, &gg, &ph, &sl, &r0, &t0};
         if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(pgrid), dim3(kThreads), args, bytes,

@@ -109,67 +109,97 @@ __device__ __forceinline__ float4 cell_velocity(const Phys &p, float h, float hu
 }
 
 // The velocities of the block's cells and of its halo cells (all threads). The block is active:
-// its own stage input in the corrector is the predictor.
+// its own stage input in the corrector is the predictor. *odd is set when a cell is not plain_cell.
 template <int STAGE>
 __device__ __forceinline__ void block_velocities(const swe_blocks_t &blocks, const swe_state_t &s,
-                                                 const Phys &p, const BlockItem &it, const BlockBuf &B) {
+                                                 const Phys &p, const BlockItem &it, const BlockBuf &B,
+                                                 volatile uint32_t *odd) {
     const uint32_t tid = threadIdx.x, i = it.b * kBlockCells + tid;
     const float h = STAGE ? s.h1[i] : s.h[i], hu = STAGE ? s.hu1[i] : s.hu[i], hv = STAGE ? s.hv1[i] : s.hv[i];
     for (uint32_t k = tid; k < it.nh; k += kThreads) {
         float hh, hhu, hhv;
         load_state<STAGE>(s, static_cast<int>(blocks.halo[it.h0 + k]), hh, hhu, hhv);
-        B.V[kBlockCells + k] = cell_velocity(p, hh, hhu, hhv);
+        const float4 c = cell_velocity(p, hh, hhu, hhv);
+        B.V[kBlockCells + k] = c;
+        if (!plain_cell(p, c)) *odd = 1u;
     }
-    B.V[tid] = cell_velocity(p, h, hu, hv);
+    const float4 c = cell_velocity(p, h, hu, hv);
+    B.V[tid] = c;
+    if (!plain_cell(p, c)) *odd = 1u;
 }
 
-// The fluxes of the block's records (all threads; records and velocities are in shared memory).
+// Record j of the block into its words. False, with nothing stored, when M cannot compute it.
+template <int STAGE, bool OPEN, class M>
+__device__ __forceinline__ bool block_edge(const swe_mesh_t &m, const swe_state_t &s, const Phys &p, const BlockItem &it,
+                                           const BlockBuf &B, uint32_t j, float dt) {
+    const float4 r = B.rec[j];
+    const float2 dz = B.dz[j];
+    const uint32_t cells = __float_as_uint(r.w), lL = cells & 0xFFFFu, lR = cells >> 16;
+    if (OPEN && M::kPlain && lR == kNoCell) return false;  // an open mesh's boundary edges: after the loop
+    const float4 L = B.V[lL];
+    float w0 = 0.0f, w1 = 0.0f, w2 = 0.0f, w3 = 0.0f, w4 = 0.0f, w5 = 0.0f;
+    bool wall = false;
+    float4 R = L;
+    if (lR != kNoCell) {
+        R = B.V[lR];
+    } else {  // a boundary edge, in the block of its left cell: the state beyond it needs the momenta
+        wall = true;
+        const uint32_t c = it.b * kBlockCells + lL;
+        const float hu = STAGE ? s.hu1[c] : s.hu[c], hv = STAGE ? s.hv1[c] : s.hv[c];
+        if (OPEN) {
+            const int cR = m.tile_cr[it.e0 + j];
+            uint32_t kind = kOpenWall;
+            float value = 0.0f, hG, huG, hvG;
+            boundary_state(m, p, cR, L.x, hu, hv, r.x, r.y, hG, huG, hvG, kind, value);
+            if (!(L.x < p.dry_tol && hG < p.dry_tol) || open_forced(kind, value)) {
+                if (!edge_words<true, M>(p, cR, r.x, r.y, r.z, dz.x, dz.y, L.x, hu, hv, hG, huG, hvG, w0, w1, w2, w3, w4,
+                                         w5, kind, value))
+                    return false;
+                if (cR < -1) tally_open(s.open_vol, static_cast<uint32_t>(-2 - cR), (0.5f * dt) * w0);
+            }
+        } else {
+            float huR, hvR;
+            wall_mirror(hu, hv, r.x, r.y, huR, hvR);
+            const float twice = 2.0f * L.x;
+            R.y = twice * huR * L.w;
+            R.z = twice * hvR * L.w;
+            if (!(L.x > p.dry_tol)) R.y = R.z = 0.0f;
+        }
+    }
+    if (!(OPEN && wall) && !(L.x < p.dry_tol && R.x < p.dry_tol)) {
+        FaceFlux f = face_flux_from_vel<M, true>(p, r.x, r.y, dz, pr(L.x, R.x), pr(L.y, R.y), pr(L.z, R.z),
+                                                    pr(L.w, R.w));
+        if (!f.plain) return false;
+        if (wall) f.Fh = 0.0f;  // a wall passes no mass
+        flux_words(p, r.x, r.y, r.z, pr(L.x, R.x), f.hs, f.Fh, f.Fhn, f.Fht, f.smax, w0, w1, w2, w3, w4, w5);
+    }
+    B.rec[j] = make_float4(w0, w1, w2, w5);
+    B.dz[j] = make_float2(w3, w4);
+    return true;
+}
+
+// The fluxes of the block's records (all threads; records and velocities are in shared memory). odd: a cell is out
+// of the branch-free operations' range (plain_cell), so every edge takes the IEEE ones; else those edges
+// whose numerators are, once more after the loop. again: a zeroed word per thread in shared memory (not a
+// register of the loop).
 template <int STAGE, bool OPEN>
 __device__ __forceinline__ void block_fluxes(const swe_mesh_t &m, const swe_state_t &s, const Phys &p,
-                                             const BlockItem &it, const BlockBuf &B, float dt) {
-    for (uint32_t j = threadIdx.x; j < it.ne; j += kThreads) {
-        const float4 r = B.rec[j];
-        const float2 dz = B.dz[j];
-        const uint32_t cells = __float_as_uint(r.w), lL = cells & 0xFFFFu, lR = cells >> 16;
-        const float4 L = B.V[lL];
-        float w0 = 0.0f, w1 = 0.0f, w2 = 0.0f, w3 = 0.0f, w4 = 0.0f, w5 = 0.0f;
-        bool wall = false;
-        float4 R = L;
-        if (lR != kNoCell) {
-            R = B.V[lR];
-        } else {  // a boundary edge, in the block of its left cell: the state beyond it needs the momenta
-            wall = true;
-            const uint32_t c = it.b * kBlockCells + lL;
-            const float hu = STAGE ? s.hu1[c] : s.hu[c], hv = STAGE ? s.hv1[c] : s.hv[c];
-            if (OPEN) {
-                const int cR = m.tile_cr[it.e0 + j];
-                uint32_t kind = kOpenWall;
-                float value = 0.0f, hG, huG, hvG;
-                boundary_state(m, p, cR, L.x, hu, hv, r.x, r.y, hG, huG, hvG, kind, value);
-                if (!(L.x < p.dry_tol && hG < p.dry_tol) || open_forced(kind, value)) {
-                    edge_words<true>(p, cR, r.x, r.y, r.z, dz.x, dz.y, L.x, hu, hv, hG, huG, hvG, w0, w1, w2, w3, w4,
-                                     w5, kind, value);
-                    if (cR < -1) tally_open(s.open_vol, static_cast<uint32_t>(-2 - cR), (0.5f * dt) * w0);
-                }
-            } else {
-                float huR, hvR;
-                wall_mirror(hu, hv, r.x, r.y, huR, hvR);
-                const float twice = 2.0f * L.x;
-                R.y = twice * huR * L.w;
-                R.z = twice * hvR * L.w;
-                if (!(L.x > p.dry_tol)) R.y = R.z = 0.0f;
-            }
+                                             const BlockItem &it, const BlockBuf &B, float dt, bool odd,
+                                             uint32_t *again) {
+    const uint32_t tid = threadIdx.x;
+    if (!odd) {
+        for (uint32_t j = tid; j < it.ne; j += kThreads)
+            if (!block_edge<STAGE, OPEN, PlainOps>(m, s, p, it, B, j, dt)) again[tid] |= 1u << (j / kThreads);
+    } else {
+        again[tid] = 0xFFFFFFFFu;
+    }
+    uint32_t rounds = again[tid];  // at most 32: the launch refuses larger blocks
+    if (rounds) {
+        again[tid] = 0u;
+        for (; rounds; rounds &= rounds - 1u) {
+            const uint32_t j = tid + (__ffs(rounds) - 1) * kThreads;
+            if (j < it.ne) block_edge<STAGE, OPEN, IeeeOps>(m, s, p, it, B, j, dt);
         }
-        if (!(OPEN && wall) && !(L.x < p.dry_tol && R.x < p.dry_tol)) {
-            float2 hs;
-            float Fh, Fhn, Fht, smax;
-            face_flux_from_vel(p, r.x, r.y, dz, pr(L.x, R.x), pr(L.y, R.y), pr(L.z, R.z), pr(L.w, R.w), hs, Fh, Fhn,
-                               Fht, smax);
-            if (wall) Fh = 0.0f;  // a wall passes no mass
-            flux_words(p, r.x, r.y, r.z, pr(L.x, R.x), hs, Fh, Fhn, Fht, smax, w0, w1, w2, w3, w4, w5);
-        }
-        B.rec[j] = make_float4(w0, w1, w2, w5);
-        B.dz[j] = make_float2(w3, w4);
     }
 }
 

@@ -244,7 +244,7 @@ int swe_apply_sources(const swe_mesh_t *mesh, const swe_state_t *state, const sw
                                                       static_cast<int>(params->compensated));
     int rc = check_launch();
     if (rc) return rc;
-    source_bound_kernel<<<grid, kThreads, 0, stream>>>(*mesh, *state, *sources, Phys{params->g, params->dry_tol}, params->cfl);
+    source_bound_kernel<<<grid, kThreads, 0, stream>>>(*mesh, *state, *sources, make_phys(params->g, params->dry_tol), params->cfl);
     return check_launch();
 }
 
@@ -273,7 +273,7 @@ int swe_cfl_prologue(const swe_mesh_t *mesh, const swe_state_t *state, const swe
     rc = set_smem(cfl_prologue_kernel, bytes);
     if (rc) return rc;
     const uint32_t grid = (params->grid == 0u || params->grid > mesh->n_blocks) ? mesh->n_blocks : params->grid;
-    cfl_prologue_kernel<<<grid, kThreads, bytes, stream>>>(*mesh, *state, Phys{params->g, params->dry_tol}, params->cfl);
+    cfl_prologue_kernel<<<grid, kThreads, bytes, stream>>>(*mesh, *state, make_phys(params->g, params->dry_tol), params->cfl);
     return check_launch();
 }
 

@@ -21,8 +21,7 @@
 // a source's wave speeds are at most u + 2c on its whole perimeter.
 // Bound: instruction issue (a steady 75-80 % of the slots; DRAM and L2 stay below 20 % of their peaks), then a
 // phase's last microseconds. Measured, one step (staged stage kernels and dilation before -> now): 600k cells
-// all wet 101 -> 82 us, 260k cells 44 % active 35 -> 28 us, 1.2M cells with rain 245 -> 194 us (the sources 40
-// -> 28 of them). With blocks dealt to CTAs in turn instead of taken, a phase of the first waits 15 us for
+// all wet 105 -> 81 us, 260k cells 44 % active 33.5 -> 21.5 us. With blocks dealt to CTAs in turn instead of taken, a phase of the first waits 15 us for
 // its last CTA (49 us instead of 41.7), and one of the second takes 16 us instead of 13.
 //
 // Every barrier and staged-data wait is bounded, as in the other kernels. The results
@@ -37,9 +36,9 @@
 
 namespace swe {
 
-// CTAs an SM must hold: 48 registers a thread. All wet 600k: 59.9 ms with 5, 62.8 with 4 (64 registers, too few
-// warps), 67.0 with 6 (40 registers spill).
-constexpr int kDenseMinCtas = 5;
+// CTAs an SM must hold: with 4, 64 registers a thread and no spills (600k cells all wet 80.7 us a step, 260k cells
+// 44 % active 21.2); with 5, 48 registers (82.7 and 22.5); 6 spill more than the warps bring.
+constexpr int kDenseMinCtas = 4;
 
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu;
 constexpr uint32_t kTakenCap = 512;  // blocks a CTA computes besides its first in one step
@@ -50,9 +49,11 @@ struct DenseShared {
     uint32_t taken[kTakenCap];  // the blocks computed besides the first in this step
     uint32_t n_taken;
     uint32_t candidate;  // the block to look at next (kNoBlock: none left)
+    uint32_t odd;       // a cell of the block is out of the branch-free operations' range
+    uint32_t again[kThreads];  // block_fluxes
     uint32_t active;    // the first block is active this step
     uint32_t red[2 * kThreads / 32];
-    int flag[2];
+    int flag[3];
     uint32_t epoch0;
 };
 
@@ -192,7 +193,7 @@ __device__ bool dense_phase(const swe_mesh_t &m, const swe_blocks_t &blocks, con
                     if (OPEN) sh.first.dt = active ? dense_dt(s, it->inst, step, epoch) : 0u;
                 }
             }
-            block_velocities<STAGE>(blocks, s, p, *it, B);
+            block_velocities<STAGE>(blocks, s, p, *it, B, &sh.odd);
         }
         // the last warp finds the next block while this one's records arrive
         if (last_warp) {
@@ -223,7 +224,7 @@ __device__ bool dense_phase(const swe_mesh_t &m, const swe_blocks_t &blocks, con
         }
         if (go) {
             st.staged = false;  // the words go over the records
-            block_fluxes<STAGE, OPEN>(m, s, p, *it, B, __uint_as_float(it->dt));
+            block_fluxes<STAGE, OPEN>(m, s, p, *it, B, __uint_as_float(it->dt), sh.odd != 0u, sh.again);
         }
         if (early && tid == kThreads - 32u) {  // in the last warp, which has the fewest records
             if (!OPEN) sh.first.dt = go ? dense_dt(s, it->inst, step, epoch) : 0u;
@@ -252,6 +253,7 @@ __device__ bool dense_phase(const swe_mesh_t &m, const swe_blocks_t &blocks, con
         } else if (early && !go && tid == 0) {
             sh.first.dt = 0u;
         }
+        if (tid == 0) sh.odd = 0u;
         // the shared memory is refilled by bulk copies
         fence_proxy_async();
         __syncthreads();
@@ -275,7 +277,9 @@ __global__ void __launch_bounds__(kThreads, kDenseMinCtas)
     const BlockBuf B = block_buf(smem, block_plan(m.max_tile_edges, blocks.max_halo, m.max_blk_slots));
     CountSync g{s.sync, 0u};  // the launch zeroes the counter before the kernel starts
     const uint32_t tid = threadIdx.x;
+    sh.again[tid] = 0u;
     if (tid == 0) {
+        sh.odd = 0u;
         mbar_init(B.bar, 1u);
         fence_barrier_init();
         sh.epoch0 = *reinterpret_cast<volatile uint32_t *>(s.sched + kSchedEpoch);  // before any CTA's first barrier
@@ -296,8 +300,6 @@ __global__ void __launch_bounds__(kThreads, kDenseMinCtas)
         if (!(ok = dense_phase<0, COMP, CLAMP, OPEN>(m, blocks, s, p, cfl, B, sh, st, computed, step, epoch, all, src)))
             break;
         if (!(ok = count_sync(g, sh.flag, nothing))) break;
-        // no instance runs this step: the steps left do nothing either (see persistent_steps_kernel)
-        if (*reinterpret_cast<volatile uint32_t *>(s.sched + kSchedIdle) == epoch) break;
         // the predictor's counter, whose phase is over, for the next step
         if (blockIdx.x == 0 && tid == 0) s.sched[kSchedTake] = 0u;
         if (!(ok = dense_phase<1, COMP, CLAMP, OPEN>(m, blocks, s, p, cfl, B, sh, st, computed, step, epoch, all, src)))
@@ -335,7 +337,9 @@ __global__ void __launch_bounds__(kThreads, kDenseMinCtas)
                 if (done) sched[kSchedIdle] = next_epoch;
             }
         };
-        if (!(ok = count_sync(g, sh.flag, control))) break;
+        if (!(ok = count_sync(g, sh.flag, control, s.sched + kSchedIdle))) break;
+        // no instance ran this step: the steps left do nothing either (see persistent_steps_kernel)
+        if (static_cast<uint32_t>(sh.flag[2]) == epoch) break;
     }
     if (st.in_flight) mbar_wait(B.bar, st.phase);
     if (tid == 0) {
@@ -363,7 +367,7 @@ int launch_dense(const swe_mesh_t *m, const swe_blocks_t *k, const swe_state_t *
     const uint32_t grid = (p->grid == 0u || p->grid > fit) ? fit : p->grid;
     // the barrier's arrival counter (at most four barriers a step) stays below 2^32
     if (4ull * n_steps * grid >= (1ull << 32)) return SWE_ERR_TOO_LARGE;
-    Phys ph{p->g, p->dry_tol};
+    Phys ph = make_phys(p->g, p->dry_tol);
     float cfl = p->cfl;
     int all_active = p->active_set ? 0 : 1;
     swe_mesh_t mm = *m;
@@ -408,7 +412,8 @@ int swe_configure_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, int
     if (!mesh_ok(mesh) || !blocks_ok(mesh, blocks) || !blocks_per_sm) return SWE_ERR_ARGUMENT;
     *blocks_per_sm = 0;
     const size_t bytes = block_bytes(mesh, blocks);
-    if (bytes > kMaxSmem || kBlockCells + blocks->max_halo >= kNoCell) return SWE_OK;
+    if (bytes > kMaxSmem || kBlockCells + blocks->max_halo >= kNoCell || mesh->max_tile_edges > 32u * kThreads)
+        return SWE_OK;
     const int rc = set_smem(dense_steps_kernel<true, false, false>, bytes);
     if (rc) return rc;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, dense_steps_kernel<true, false, false>, kThreads,
@@ -427,7 +432,8 @@ int swe_steps_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, const s
         (!sources->hscale || !sources->knot_ptr || !sources->knot_t || !sources->knot_q || sources->n_hydro == 0u))
         return SWE_ERR_ARGUMENT;
     if (mesh->max_sub_edges > 2047u || mesh->max_sub_slots > 2047u || mesh->n_inst > 1023u ||
-        mesh->n_blocks > (1u << 23) || kBlockCells + blocks->max_halo >= kNoCell)
+        mesh->n_blocks > (1u << 23) || kBlockCells + blocks->max_halo >= kNoCell ||
+        mesh->max_tile_edges > 32u * kThreads)
         return SWE_ERR_TOO_LARGE;
     if (n_steps == 0u) return SWE_OK;
     return mesh->n_open ? dispatch_dense<true>(mesh, blocks, state, params, sources, n_steps, stream)

@@ -93,13 +93,15 @@ struct CountSync {
     uint32_t target;  // arrivals that complete the next barrier
 };
 
+// word != nullptr: its value, read beside the arrival (one round trip for both), goes to flag[2].
 template <typename F>
-__device__ __forceinline__ bool count_sync(CountSync &g, int *flag, F after) {
+__device__ __forceinline__ bool count_sync(CountSync &g, int *flag, F after, const uint32_t *word = nullptr) {
     fence_proxy_async_global();
     __syncthreads();
     g.target += gridDim.x;
     if (threadIdx.x == 0) {
         flag[1] = 1;
+        if (word) flag[2] = static_cast<int>(*reinterpret_cast<const volatile uint32_t *>(word));
         const uint32_t old = atom_add_acq_rel_gpu(g.count, 1u);
         flag[0] = old + 1u == g.target ? 1 : 0;
         if (old + 1u != g.target) {

@@ -75,6 +75,14 @@ __global__ void open_ghost_kernel(const float *cases, const uint32_t *cond, floa
     }
 }
 
+__global__ void plain_math_kernel(const float *a, const float *b, float *out, uint32_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        out[i] = plain_rcp(b[i]);
+        out[static_cast<size_t>(n) + i] = plain_div(a[i], b[i]);
+        out[2ull * n + i] = plain_sqrt(b[i]);
+    }
+}
+
 // One bounded wait for instance 0's published dt pair (the seats' wait in the
 // persistent kernel): the dt bits, or 0 and error bit 4 after the wait limit.
 __global__ void dt_wait_probe_kernel(swe_state_t s, uint32_t epoch, uint32_t *out) {
@@ -124,12 +132,16 @@ int swe_inv_pow43(const float *x, float *out, uint32_t n, swe_stream_t stream) {
     return check_launch();
 }
 
+int swe_plain_math_probe(const float *a, const float *b, float *out, uint32_t n, swe_stream_t stream) {
+    if (!a || !b || !out || n == 0u) return SWE_ERR_ARGUMENT;
+    plain_math_kernel<<<min((n + 255u) / 256u, 4096u), 256, 0, stream>>>(a, b, out, n);
+    return check_launch();
+}
+
 int swe_open_ghost_probe(const float *cases, const uint32_t *cond, float *results, uint32_t n, float g,
                          float dry_tol, swe_stream_t stream) {
     if (!cases || !cond || !results || n == 0u) return SWE_ERR_ARGUMENT;
-    Phys p;
-    p.g = g;
-    p.dry_tol = dry_tol;
+    const Phys p = make_phys(g, dry_tol);
     open_ghost_kernel<<<min((n + 255u) / 256u, 4096u), 256, 0, stream>>>(cases, cond, results, n, p);
     return check_launch();
 }

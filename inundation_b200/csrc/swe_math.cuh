@@ -10,6 +10,7 @@
 // value the reference admits. GLSL min/max/clamp are written with their
 // specified comparisons: min(x,y) = y<x ? y : x, max(x,y) = x<y ? y : x.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 namespace swe {
@@ -21,7 +22,13 @@ constexpr float kDtSentinel = 1e30f;
 struct Phys {
     float g;
     float dry_tol;
+    float root_g;  // sqrt(g)
+    bool plain;    // g and dry_tol leave the flux's operands in the range of the branch-free operations
 };
+
+inline Phys make_phys(float g, float dry_tol) {
+    return Phys{g, dry_tol, sqrtf(g), g >= 0.0625f && g <= 1e3f && dry_tol >= 1e-9f && dry_tol <= 1e3f};
+}
 
 __device__ __forceinline__ float fmaf_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float gmin(float x, float y) { return (y < x) ? y : x; }
@@ -76,7 +83,7 @@ __device__ __forceinline__ void hllc_speeds(const Phys &p, float hL, float unL, 
                                             float &SRo) {
     const float sqL = sqrtf(gmax(hL, 0.0f));
     const float sqR = sqrtf(gmax(hR, 0.0f));
-    const float root_g = sqrtf(p.g);  // loop-invariant: hoisted out of the callers' edge loops
+    const float root_g = p.root_g;
     const float cL = root_g * sqL;
     const float cR = root_g * sqR;
     const float den = sqL + sqR;
@@ -107,7 +114,7 @@ __device__ __forceinline__ void hllc_speeds_fast(const Phys &p, float hL, float 
                                                  float &SRo) {
     const float sqL = sqrtf(gmax(hL, 0.0f));
     const float sqR = sqrtf(gmax(hR, 0.0f));
-    const float root_g = sqrtf(p.g);  // loop-invariant: hoisted out of the callers' edge loops
+    const float root_g = p.root_g;
     const float cL = root_g * sqL;
     const float cR = root_g * sqR;
     const float den = sqL + sqR;
@@ -191,6 +198,48 @@ __device__ __forceinline__ void wall_mirror(float huL, float hvL, float nx, floa
     hvR = fmaf_rn(twice, ny, hvL);
 }
 
+// -- correctly rounded quotients and roots without branches ------------------------------------------
+// Reciprocal, quotient and square root from the hardware's approximations (PTX rcp.approx and
+// rsqrt.approx, about one ulp) by Newton steps in fused multiply-adds, ended by the correction
+// that Markstein proved to round correctly (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: from the correctly rounded
+// reciprocal y of b and a quotient q within one ulp, fma(fma(-b, q, a), y, q) is the correctly
+// rounded a / b; likewise for the root with half its reciprocal). They equal the IEEE operations
+// for operands far from under- and overflow, which the caller checks: x and b in [2^-80, 2^62],
+// a quotient's numerator 0 or in that range (a zero quotient may come out with the other sign).
+// The compiler's own operations check every operand and branch, so several in a row cannot
+// overlap; these can, and two of a kind share the paired instructions.
+constexpr float kPlainMin = 8.271806125530277e-25f;  // 2^-80
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float plain_rcp(float b) {
+    const float y = rcp_approx(b);
+    return fmaf_rn(fmaf_rn(-b, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float plain_div(float a, float b) {
+    const float y = plain_rcp(b);
+    const float q = a * y;
+    return fmaf_rn(fmaf_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ float plain_sqrt(float x) {  // 0 for 0
+    const float y = rsqrt_approx(x);
+    float g = x * y, h = 0.5f * y;
+    const float r = fmaf_rn(-h, g, 0.5f);
+    g = fmaf_rn(g, r, g);
+    h = fmaf_rn(h, r, h);
+    const float root = fmaf_rn(fmaf_rn(-g, g, x), h, g);
+    return x > 0.0f ? root : 0.0f;
+}
+
 // -- open boundaries (flux.py:187-294) ----------------------------------------------------------
 // Open edge k has cR = -2 - k; its condition is the word pair (kind, value bits).
 constexpr uint32_t kOpenWall = 0u, kOpenFree = 1u, kOpenNormal = 2u, kOpenStage = 3u, kOpenInflow = 4u;
@@ -210,7 +259,7 @@ __device__ __forceinline__ float cbrt_newton(float x) {
 // Depth beyond an inflow edge of discharge q per unit width: the root of
 // -q/hG + 2 sqrt(g hG) = riemann (the outgoing characteristic), by Newton in s = sqrt(hG).
 __device__ __forceinline__ float inflow_depth(const Phys &p, float q, float riemann) {
-    const float root_g = sqrtf(p.g);
+    const float root_g = p.root_g;
     float s = gmax(cbrt_newton(q / (2.0f * root_g)), riemann / (2.0f * root_g));
     for (int k = 0; k < kOpenNewtonSteps; ++k) {
         const float f = 2.0f * root_g * s - q / (s * s) - riemann;

@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ TiledShared<kPersistThreads> sh;
     __shared__ SeatShared ss;
-    __shared__ int flag[2];
+    __shared__ int flag[3];
     __shared__ uint32_t epoch0;
     CountSync g{s.sync, 0u};  // the launch zeroes the counter before the kernel starts
     if (threadIdx.x == 0) {
@@ -616,10 +616,6 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
                                                       src.count != 0u && !fused)))
             break;
         if (!(ok = count_sync(g, flag, nothing))) break;
-        // No instance runs this step (every window is done): the steps left do nothing either, 5 us each on a
-        // small mesh (8 fixed steps of 2048 cells took 1.02 ms of a 200-step launch). The last
-        // step's control wrote the word before its CTA came to the barrier just passed, so every CTA sees it.
-        if ((idle = *reinterpret_cast<volatile uint32_t *>(s.sched + kSchedIdle) == epoch)) break;
         if (!(ok = seat_corrector<COMP, CLAMP, OPEN>(m, s, p, cfl, smem, sh, ss, ph, computed, step, epoch, all, src,
                                                      fused)))
             break;
@@ -648,10 +644,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
                 __syncthreads();  // the bounds land before step_control reads them
             }
             bool runs = false, out = false;
-            if (fused && !all)
+            if (fused && !all) {
                 for (uint32_t k = threadIdx.x; k < src.count; k += blockDim.x)
                     out |= s.marks[2u * (__ldg(src.cells + k) >> 8)] != next_epoch;
-            out = __syncthreads_or(out) != 0;
+                out = __syncthreads_or(out) != 0;
+            }
             for (uint32_t i = threadIdx.x; i < m.n_inst; i += blockDim.x) {
                 const uint32_t dt = step_control(s.ctrl + i, s.dt_buf + kDtWords * i, 1);
                 runs |= dt != 0u;
@@ -680,7 +677,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         };
         // The step control runs after the release, the others wait for its dt pairs
         // only where they need them.
-        if (!(ok = count_sync(g, flag, control))) break;
+        if (!(ok = count_sync(g, flag, control, s.sched + kSchedIdle))) break;
+        // No instance ran this step (every window is done): the steps left do nothing either, 5 us each on a
+        // small mesh (8 fixed steps of 2048 cells took 1.02 ms of a 200-step launch). The control of the step
+        // before wrote the word, so every CTA finds it here; read earlier, it would delay every corrector.
+        if ((idle = static_cast<uint32_t>(flag[2]) == epoch)) break;
         // the hand-over reads the last step's dt and the lists its control zeroes
         if (last_step && !(ok = count_sync(g, flag, nothing))) break;
     }
@@ -710,7 +711,7 @@ int launch_persistent(const swe_mesh_t *m, const swe_state_t *s, const swe_param
     if (4ull * m->n_blocks > static_cast<uint64_t>(grid) * (1u + kExtraCap)) return SWE_ERR_TOO_LARGE;
     // the barrier's arrival counter (at most four barriers a step, one more at the end) stays below 2^32
     if ((4ull * n_steps + 1ull) * grid >= (1ull << 32)) return SWE_ERR_TOO_LARGE;
-    Phys ph{p->g, p->dry_tol};
+    Phys ph = make_phys(p->g, p->dry_tol);
     float cfl = p->cfl;
     int all_active = p->active_set ? 0 : 1;
     swe_mesh_t mm = *m;

@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kTileThreads, 8)
 template <int STAGE, bool COMP, bool CLAMP, bool OPEN>
 int launch_stage(const swe_mesh_t *m, const swe_state_t *s, const swe_params_t *p, cudaStream_t st,
                  float *sums = nullptr) {
-    const Phys ph{p->g, p->dry_tol};
+    const Phys ph = make_phys(p->g, p->dry_tol);
     if (p->kernel == 3u) {
         if (!m->blk_lcsr || !m->blk_lcsr_ptr) return SWE_ERR_ARGUMENT;
         auto kern = stage_staged_kernel<STAGE, COMP, CLAMP, OPEN>;

@@ -185,6 +185,9 @@ class ResidentEngine:
             "dz": torch.stack([t["tile_dzl"], t["tile_dzr"]], dim=1),
             "halo": self._dev(B.halo), "halo_ptr": self._dev(_i32(B.halo_ptr)),
         }
+        dz = self._blocks_t["dz"]
+        if not bool(((dz >= 0.0) & (dz <= 2.0**19)).all()):
+            return  # not the face steps of a bed: the kernel's range check relies on them
         # every cell's perimeter, rounded up by more than the order of summing its edges can change
         own = (local.view(torch.int32) & 0xFFFF) < B.tile_cells  # records in the tile of their left cell: each edge once
         inner = own & (t["tile_cr"] >= 0)
