@@ -17,8 +17,9 @@
 //   cell1       the Heun average and the corrector's cell update: adjoint of
 //               the corrector sums and of the predictor state (local part)
 //   edge<1>     the corrector's edges: adjoint of the predictor state through
-//               the fluxes, gathered per cell in CSR order (no float atomics)
-//   cell0       the predictor's cell update
+//               the fluxes, gathered per cell in CSR order (no float atomics), then
+//               at once the predictor's cell update of those cells (its adjoint sums
+//               replace lsh, lshu, lshv, which only the cell itself reads)
 //   edge<0>     the predictor's edges, into the adjoint of the step's start state
 // Parameter gradients: Manning n in the cell kernels, the bed through the
 // edges' face steps dzL = max(zL, zR) - zL, dzR = max(zL, zR) - zR.
@@ -137,6 +138,10 @@ __device__ __forceinline__ void cell_reverse(const Phys &p, float dt, float A, f
 }
 
 // -- edge reverse ---------------------------------------------------------------------------------
+// The reverse's quotients are products by a reciprocal, shared where the denominator is: correctly rounded, and
+// branch-free where the denominators are in range (p.plain; all are sums of squares, or above a threshold).
+__device__ __forceinline__ float rcp_of(const Phys &p, float b) { return p.plain ? plain_rcp(b) : 1.0f / b; }
+
 __device__ __forceinline__ void safe_vel_rev(const Phys &p, float h, float q, float gu, float &gh, float &gq) {
     if (!(h > p.dry_tol) || gu == 0.0f) return;
     const float e = kFilmDepths * p.dry_tol;
@@ -144,8 +149,9 @@ __device__ __forceinline__ void safe_vel_rev(const Phys &p, float h, float q, fl
     const bool big = !(h2 < e2);  // gmax(h2, e2)
     const float D = h2 + (big ? h2 : e2);
     const float dD = big ? 4.0f * h : 2.0f * h;
-    gq += gu * 2.0f * h / D;
-    gh += gu * (2.0f * q / D - 2.0f * h * q * dD / (D * D));
+    const float inv = rcp_of(p, D);
+    gq += gu * 2.0f * h * inv;
+    gh += gu * (2.0f * q * inv - 2.0f * h * q * inv * (dD * inv));
 }
 
 __device__ __forceinline__ float wet_blend_d(const Phys &p, float h) {
@@ -228,18 +234,19 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         const float dSL = SL - SM;
         const bool dok = fabsf(dSL) > 1e-14f;
         const float d = dok ? dSL : 1e-14f;
-        const float kL = hLs * (SL - unL) / d;
+        const float inv = rcp_of(p, d);
+        const float kL = hLs * (SL - unL) * inv;
         gSL += gFh * (kL - hLs) + gFhn * (kL * SM - hLs * unL) + gFht * (kL * utL - hLs * utL);
         const float gkL = gFh * SL + gFhn * SL * SM + gFht * SL * utL;
         gSM += gFhn * SL * kL;
         ghLs += gFh * (unL - SL) + gFhn * (unL * unL + p.g * hLs - SL * unL) + gFht * (unL * utL - SL * utL);
         gunL += gFh * hLs + gFhn * (2.0f * hLs * unL - SL * hLs) + gFht * hLs * utL;
         gutL += gFht * (hLs * unL + SL * kL - SL * hLs);
-        ghLs += gkL * (SL - unL) / d;
-        gSL += gkL * hLs / d;
-        gunL -= gkL * hLs / d;
+        ghLs += gkL * (SL - unL) * inv;
+        gSL += gkL * hLs * inv;
+        gunL -= gkL * hLs * inv;
         if (dok) {
-            const float gd = -gkL * kL / d;
+            const float gd = -gkL * kL * inv;
             gSL += gd;
             gSM -= gd;
         }
@@ -247,24 +254,25 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         const float dSR = SR - SM;
         const bool dok = fabsf(dSR) > 1e-14f;
         const float d = dok ? dSR : 1e-14f;
-        const float kR = hRs * (SR - unR) / d;
+        const float inv = rcp_of(p, d);
+        const float kR = hRs * (SR - unR) * inv;
         gSR += gFh * (kR - hRs) + gFhn * (kR * SM - hRs * unR) + gFht * (kR * utR - hRs * utR);
         const float gkR = gFh * SR + gFhn * SR * SM + gFht * SR * utR;
         gSM += gFhn * SR * kR;
         ghRs += gFh * (unR - SR) + gFhn * (unR * unR + p.g * hRs - SR * unR) + gFht * (unR * utR - SR * utR);
         gunR += gFh * hRs + gFhn * (2.0f * hRs * unR - SR * hRs) + gFht * hRs * utR;
         gutR += gFht * (hRs * unR + SR * kR - SR * hRs);
-        ghRs += gkR * (SR - unR) / d;
-        gSR += gkR * hRs / d;
-        gunR -= gkR * hRs / d;
+        ghRs += gkR * (SR - unR) * inv;
+        gSR += gkR * hRs * inv;
+        gunR -= gkR * hRs * inv;
         if (dok) {
-            const float gd = -gkR * kR / d;
+            const float gd = -gkR * kR * inv;
             gSR += gd;
             gSM -= gd;
         }
     }
     if (sm_ok && gSM != 0.0f) {
-        const float gnum = gSM / den_sm, gden = -gSM * SM / den_sm;
+        const float gnum = gSM * rcp_of(p, den_sm), gden = -gnum * SM;
         gSL += gnum * (hRs * (unR - SR) + SR * hLs) + gden * hLs;
         gSR += gnum * (-SL * hRs - hLs * (unL - SL)) - gden * hRs;
         ghRs += gnum * SL * (unR - SR) + gden * (unR - SR);
@@ -301,19 +309,22 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         gcR += gSR0;
     }
     if (c_roe > 0.0f) {
-        const float t = gc_roe * 0.25f * p.g / c_roe;
+        const float t = gc_roe * 0.25f * p.g * rcp_of(p, c_roe);
         ghLs += t;
         ghRs += t;
     }
     if (roe_ok) {
-        const float gsqL = gu_roe * (unL - u_roe) / den, gsqR = gu_roe * (unR - u_roe) / den;
-        gunL += gu_roe * sqL / den;
-        gunR += gu_roe * sqR / den;
-        if (sqL > 0.0f) ghLs += gsqL * 0.5f / sqL;
-        if (sqR > 0.0f) ghRs += gsqR * 0.5f / sqR;
+        const float per = gu_roe * rcp_of(p, den);
+        const float gsqL = per * (unL - u_roe), gsqR = per * (unR - u_roe);
+        gunL += per * sqL;
+        gunR += per * sqR;
+        // the roots' derivatives: 1 / (2 sqrt h), and root_g times it for the celerities
+        if (sqL > 0.0f) ghLs += (gsqL + gcL * root_g) * 0.5f * rcp_of(p, sqL);
+        if (sqR > 0.0f) ghRs += (gsqR + gcR * root_g) * 0.5f * rcp_of(p, sqR);
+    } else {
+        if (cL > 0.0f) ghLs += gcL * 0.5f * p.g / cL;
+        if (cR > 0.0f) ghRs += gcR * 0.5f * p.g / cR;
     }
-    if (cL > 0.0f) ghLs += gcL * 0.5f * p.g / cL;
-    if (cR > 0.0f) ghRs += gcR * 0.5f * p.g / cR;
     // face-frame velocities
     float ghqnL = 0.0f, ghqtL = 0.0f, ghqnR = 0.0f, ghqtR = 0.0f;
     safe_vel_rev(p, hLs, hqnL, gunL, ghLs, ghqnL);
@@ -457,36 +468,27 @@ __device__ void adj_cell1(const swe_mesh_t &m, const swe_tape_t &T, const swe_ad
     }
 }
 
-// The predictor's cell update, reversed.
-__device__ void adj_cell0(const swe_mesh_t &m, const swe_tape_t &T, const swe_adjoint_t &a, const Phys &p, uint32_t k) {
-    const uint32_t n = m.n_blocks * kBlockCells;
-    const uint32_t count = T.count[k];
-    const Slot S = slot_of(T, k, n, m.n_blocks);
-    const float dt = __uint_as_float(T.dt[k]);
-    for (uint32_t w = blockIdx.x; w < count; w += gridDim.x) {
-        const uint32_t b = S.list[w];
-        if (threadIdx.x >= m.block_cells[b]) continue;
-        const uint32_t i = b * kBlockCells + threadIdx.x;
-        const float A = m.area[i], nm = m.n_mann[i];
-        const CellFwd c0 =
-            cell_forward(p, dt, A, nm, S.h[i], S.lo[i], S.hu[i], S.hv[i], S.s0[i], S.s0[n + i], S.s0[2 * n + i]);
-        float g_h = 0.0f, g_hu = 0.0f, g_hv = 0.0f, g_sh, g_su, g_sv, g_n = 0.0f;
-        cell_reverse(p, dt, A, nm, c0, a.lsh[i], a.lshu[i], a.lshv[i], g_h, g_hu, g_hv, g_sh, g_su, g_sv, g_n,
-                     S.h[i] < a.cut_depth, a.cut_depth);
-        a.ls[i] = g_sh;
-        a.ls[n + i] = g_su;
-        a.ls[2 * n + i] = g_sv;
-        a.lh[i] += g_h;
-        a.lhu[i] += g_hu;
-        a.lhv[i] += g_hv;
-        a.gn[i] += g_n;
-    }
+// The predictor's cell update of cell i, reversed, from the adjoint (gh, ghu, ghv) of its predictor state.
+__device__ __forceinline__ void adj_cell0(const swe_mesh_t &m, const Slot &S, const swe_adjoint_t &a, const Phys &p,
+                                          uint32_t n, uint32_t i, float dt, float gh, float ghu, float ghv) {
+    const float A = m.area[i], nm = m.n_mann[i], h = S.h[i];
+    const CellFwd c0 = cell_forward(p, dt, A, nm, h, S.lo[i], S.hu[i], S.hv[i], S.s0[i], S.s0[n + i], S.s0[2 * n + i]);
+    float g_h = 0.0f, g_hu = 0.0f, g_hv = 0.0f, g_sh, g_su, g_sv, g_n = 0.0f;
+    cell_reverse(p, dt, A, nm, c0, gh, ghu, ghv, g_h, g_hu, g_hv, g_sh, g_su, g_sv, g_n, h < a.cut_depth, a.cut_depth);
+    a.lsh[i] = g_sh;
+    a.lshu[i] = g_su;
+    a.lshv[i] = g_sv;
+    a.lh[i] += g_h;
+    a.lhu[i] += g_hu;
+    a.lhv[i] += g_hv;
+    a.gn[i] += g_n;
 }
 
 // Edge adjoints of one stage, gathered per cell in the forward's CSR order.
 // STAGE 1: the corrector (inputs: the predictor state in blocks of this step,
-// the start state elsewhere; adds into the predictor's adjoint). STAGE 0: the
-// predictor (inputs: the start state; adds into the start state's adjoint).
+// the start state elsewhere; adds into the predictor's adjoint and takes it through the
+// predictor's cell update). STAGE 0: the predictor (inputs: the start state; adds into the
+// start state's adjoint).
 template <int STAGE>
 __device__ void adj_edge(const swe_mesh_t &m, const swe_tape_t &T, const swe_adjoint_t &a, const Phys &p, uint32_t k,
                          uint32_t tag, float *G) {
@@ -494,6 +496,9 @@ __device__ void adj_edge(const swe_mesh_t &m, const swe_tape_t &T, const swe_adj
     const uint32_t cap = (m.max_sub_edges + 3u) & ~3u;
     const uint32_t n = m.n_blocks * kBlockCells;
     const Slot S = slot_of(T, k, n, m.n_blocks);
+    // the adjoint of the stage's sums
+    const float *l0 = STAGE ? a.ls : a.lsh, *l1 = STAGE ? a.ls + n : a.lshu, *l2 = STAGE ? a.ls + 2 * n : a.lshv;
+    const float dt = __uint_as_float(T.dt[k]);
     // one 64-cell tile per CTA pass: four per active block, one edge record per thread
     for (uint32_t w = blockIdx.x; w < 4u * count; w += gridDim.x) {
         const uint32_t b = S.list[w >> 2], q4 = w & 3u;
@@ -534,10 +539,8 @@ __device__ void adj_edge(const swe_mesh_t &m, const swe_tape_t &T, const swe_adj
             }
             EdgeGrad eg{};
             if (!(hL < p.dry_tol && hR < p.dry_tol)) {
-                const float lhL = actL ? a.ls[cL] : 0.0f, luL = actL ? a.ls[n + cL] : 0.0f,
-                            lvL = actL ? a.ls[2 * n + cL] : 0.0f;
-                const float lhR = actR ? a.ls[cR] : 0.0f, luR = actR ? a.ls[n + cR] : 0.0f,
-                            lvR = actR ? a.ls[2 * n + cR] : 0.0f;
+                const float lhL = actL ? l0[cL] : 0.0f, luL = actL ? l1[cL] : 0.0f, lvL = actL ? l2[cL] : 0.0f;
+                const float lhR = actR ? l0[cR] : 0.0f, luR = actR ? l1[cR] : 0.0f, lvR = actR ? l2[cR] : 0.0f;
                 eg = edge_words_rev(p, cR < 0, nx, ny, m.sub_len[e], m.sub_dzl[e], m.sub_dzr[e], hL, huL, hvL, hR,
                                     huR, hvR, lhL - lhR, luL, lvL, -luR, -lvR, a.cut_depth);
             }
@@ -554,10 +557,10 @@ __device__ void adj_edge(const swe_mesh_t &m, const swe_tape_t &T, const swe_adj
         __syncthreads();
         if (threadIdx.x < min(static_cast<uint32_t>(kTileCells), cells - q4 * kTileCells)) {
             const uint32_t i = t * kTileCells + threadIdx.x;
-            const uint32_t l0 = m.sub_lcsr_ptr[t], c0 = m.cptr[t * kTileCells];
+            const uint32_t first = m.sub_lcsr_ptr[t], c0 = m.cptr[t * kTileCells];
             float sh = 0.0f, su = 0.0f, sv = 0.0f, sz = 0.0f;
             for (uint32_t q = m.cptr[i], q1 = m.cptr[i + 1]; q < q1; ++q) {
-                const uint32_t v = m.sub_lcsr[l0 + q - c0];
+                const uint32_t v = m.sub_lcsr[first + q - c0];
                 const uint32_t j = v >> 1;
                 if (v & 1u) {
                     sh += G[3 * cap + j];
@@ -572,9 +575,7 @@ __device__ void adj_edge(const swe_mesh_t &m, const swe_tape_t &T, const swe_adj
                 }
             }
             if (STAGE == 1) {
-                a.lsh[i] += sh;
-                a.lshu[i] += su;
-                a.lshv[i] += sv;
+                adj_cell0(m, S, a, p, n, i, dt, a.lsh[i] + sh, a.lshu[i] + su, a.lshv[i] + sv);
             } else {
                 a.lh[i] += sh;
                 a.lhu[i] += su;
@@ -596,18 +597,20 @@ __global__ void __launch_bounds__(kThreads)
     adj_cell1(m, T, a, p, k, tag);
 }
 
-__global__ void __launch_bounds__(kThreads) adj_cell0_kernel(swe_mesh_t m, swe_tape_t T, swe_adjoint_t a, Phys p, uint32_t k) {
-    adj_cell0(m, T, a, p, k);
-}
+// The edge phases are bound by latency: a chain of loads (list, tile, records, states) and some 500 dependent
+// operations per tile. 64 registers let 592 CTAs be resident, one tile each at 250k cells with 14 % active (where
+// 100 registers took two rounds): edge<1>, with the predictor's cell update, 21.6 + 6.9 -> 14.2 us, edge<0>
+// 20.8 -> 9.7 us; the shared branch-free reciprocals are about half of the gain.
+constexpr int kAdjEdgeCtas = 4;
 
 template <int STAGE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kAdjEdgeCtas)
     adj_edge_kernel(swe_mesh_t m, swe_tape_t T, swe_adjoint_t a, Phys p, uint32_t k, uint32_t tag) {
     extern __shared__ float4 smem4[];
     adj_edge<STAGE>(m, T, a, p, k, tag, reinterpret_cast<float *>(smem4));
 }
 
-// The reverse of a whole segment in one cooperative launch: the five phases of
+// The reverse of a whole segment in one cooperative launch: the four phases of
 // every step, slot by slot from the last, separated by grid barriers instead of
 // kernel boundaries. A barrier wait past its bound sets a.sync[40] and stops.
 __global__ void __launch_bounds__(kThreads)
@@ -629,8 +632,6 @@ __global__ void __launch_bounds__(kThreads)
         adj_cell1(m, T, a, p, kk, tag);
         if (!(ok = grid_sync(g, flag, nothing))) break;
         adj_edge<1>(m, T, a, p, kk, tag, G);
-        if (!(ok = grid_sync(g, flag, nothing))) break;
-        adj_cell0(m, T, a, p, kk);
         if (!(ok = grid_sync(g, flag, nothing))) break;
         adj_edge<0>(m, T, a, p, kk, tag, G);
         ok = grid_sync(g, flag, nothing);
@@ -785,8 +786,6 @@ int swe_adjoint_segment(const swe_mesh_t *mesh, const swe_params_t *params, cons
         adj_cell1_kernel<<<grid, kThreads, 0, stream>>>(*mesh, *tape, *adj, ph, kk, tag);
         if ((rc = check_launch())) return rc;
         adj_edge_kernel<1><<<grid, kThreads, bytes, stream>>>(*mesh, *tape, *adj, ph, kk, tag);
-        if ((rc = check_launch())) return rc;
-        adj_cell0_kernel<<<grid, kThreads, 0, stream>>>(*mesh, *tape, *adj, ph, kk);
         if ((rc = check_launch())) return rc;
         adj_edge_kernel<0><<<grid, kThreads, bytes, stream>>>(*mesh, *tape, *adj, ph, kk, tag);
         if ((rc = check_launch())) return rc;

@@ -209,6 +209,14 @@ int launch_handover(const swe_mesh_t *m, const swe_state_t *s, const swe_params_
     return check_launch();
 }
 
+// A few sources in one CTA: the increments, then the bounds, without a launch between them.
+__global__ void __launch_bounds__(kThreads)
+    source_few_kernel(swe_mesh_t m, swe_state_t s, swe_sources_t src, Phys p, float cfl, int comp) {
+    source_apply(m, s, src, p.dry_tol, comp, threadIdx.x, kThreads);
+    __syncthreads();
+    source_bound_cta(m, s, src, p, cfl);
+}
+
 inline size_t cfl_smem_bytes(uint32_t max_tile_edges) { return ((max_tile_edges + 3u) & ~3u) * sizeof(float); }
 
 inline bool items_fit(const swe_mesh_t *m) {
@@ -239,6 +247,13 @@ int swe_apply_sources(const swe_mesh_t *mesh, const swe_state_t *state, const sw
     if (sources->hydro &&
         (!sources->hscale || !sources->knot_ptr || !sources->knot_t || !sources->knot_q || sources->n_hydro == 0u))
         return SWE_ERR_ARGUMENT;
+    // One launch instead of two up to a CTA's worth of sources, 8 lanes each for the bounds (one source: 4.2 us
+    // against 3.2 + 4.5); more take the passes, whose threads spread over the GPU.
+    if (sources->count <= kThreads) {
+        source_few_kernel<<<1, kThreads, 0, stream>>>(*mesh, *state, *sources, make_phys(params->g, params->dry_tol),
+                                                      params->cfl, static_cast<int>(params->compensated));
+        return check_launch();
+    }
     const uint32_t grid = min((sources->count + kThreads - 1) / kThreads, 148u * 16u);
     source_apply_kernel<<<grid, kThreads, 0, stream>>>(*mesh, *state, *sources, params->dry_tol,
                                                       static_cast<int>(params->compensated));
