@@ -138,10 +138,6 @@ __device__ __forceinline__ void cell_reverse(const Phys &p, float dt, float A, f
 }
 
 // -- edge reverse ---------------------------------------------------------------------------------
-// The reverse's quotients are products by a reciprocal, shared where the denominator is: correctly rounded, and
-// branch-free where the denominators are in range (p.plain; all are sums of squares, or above a threshold).
-__device__ __forceinline__ float rcp_of(const Phys &p, float b) { return p.plain ? plain_rcp(b) : 1.0f / b; }
-
 __device__ __forceinline__ void safe_vel_rev(const Phys &p, float h, float q, float gu, float &gh, float &gq) {
     if (!(h > p.dry_tol) || gu == 0.0f) return;
     const float e = kFilmDepths * p.dry_tol;
@@ -149,9 +145,8 @@ __device__ __forceinline__ void safe_vel_rev(const Phys &p, float h, float q, fl
     const bool big = !(h2 < e2);  // gmax(h2, e2)
     const float D = h2 + (big ? h2 : e2);
     const float dD = big ? 4.0f * h : 2.0f * h;
-    const float inv = rcp_of(p, D);
-    gq += gu * 2.0f * h * inv;
-    gh += gu * (2.0f * q * inv - 2.0f * h * q * inv * (dD * inv));
+    gq += gu * 2.0f * h / D;
+    gh += gu * (2.0f * q / D - 2.0f * h * q * dD / (D * D));
 }
 
 __device__ __forceinline__ float wet_blend_d(const Phys &p, float h) {
@@ -234,19 +229,18 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         const float dSL = SL - SM;
         const bool dok = fabsf(dSL) > 1e-14f;
         const float d = dok ? dSL : 1e-14f;
-        const float inv = rcp_of(p, d);
-        const float kL = hLs * (SL - unL) * inv;
+        const float kL = hLs * (SL - unL) / d;
         gSL += gFh * (kL - hLs) + gFhn * (kL * SM - hLs * unL) + gFht * (kL * utL - hLs * utL);
         const float gkL = gFh * SL + gFhn * SL * SM + gFht * SL * utL;
         gSM += gFhn * SL * kL;
         ghLs += gFh * (unL - SL) + gFhn * (unL * unL + p.g * hLs - SL * unL) + gFht * (unL * utL - SL * utL);
         gunL += gFh * hLs + gFhn * (2.0f * hLs * unL - SL * hLs) + gFht * hLs * utL;
         gutL += gFht * (hLs * unL + SL * kL - SL * hLs);
-        ghLs += gkL * (SL - unL) * inv;
-        gSL += gkL * hLs * inv;
-        gunL -= gkL * hLs * inv;
+        ghLs += gkL * (SL - unL) / d;
+        gSL += gkL * hLs / d;
+        gunL -= gkL * hLs / d;
         if (dok) {
-            const float gd = -gkL * kL * inv;
+            const float gd = -gkL * kL / d;
             gSL += gd;
             gSM -= gd;
         }
@@ -254,25 +248,24 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         const float dSR = SR - SM;
         const bool dok = fabsf(dSR) > 1e-14f;
         const float d = dok ? dSR : 1e-14f;
-        const float inv = rcp_of(p, d);
-        const float kR = hRs * (SR - unR) * inv;
+        const float kR = hRs * (SR - unR) / d;
         gSR += gFh * (kR - hRs) + gFhn * (kR * SM - hRs * unR) + gFht * (kR * utR - hRs * utR);
         const float gkR = gFh * SR + gFhn * SR * SM + gFht * SR * utR;
         gSM += gFhn * SR * kR;
         ghRs += gFh * (unR - SR) + gFhn * (unR * unR + p.g * hRs - SR * unR) + gFht * (unR * utR - SR * utR);
         gunR += gFh * hRs + gFhn * (2.0f * hRs * unR - SR * hRs) + gFht * hRs * utR;
         gutR += gFht * (hRs * unR + SR * kR - SR * hRs);
-        ghRs += gkR * (SR - unR) * inv;
-        gSR += gkR * hRs * inv;
-        gunR -= gkR * hRs * inv;
+        ghRs += gkR * (SR - unR) / d;
+        gSR += gkR * hRs / d;
+        gunR -= gkR * hRs / d;
         if (dok) {
-            const float gd = -gkR * kR * inv;
+            const float gd = -gkR * kR / d;
             gSR += gd;
             gSM -= gd;
         }
     }
     if (sm_ok && gSM != 0.0f) {
-        const float gnum = gSM * rcp_of(p, den_sm), gden = -gnum * SM;
+        const float gnum = gSM / den_sm, gden = -gSM * SM / den_sm;
         gSL += gnum * (hRs * (unR - SR) + SR * hLs) + gden * hLs;
         gSR += gnum * (-SL * hRs - hLs * (unL - SL)) - gden * hRs;
         ghRs += gnum * SL * (unR - SR) + gden * (unR - SR);
@@ -309,22 +302,19 @@ __device__ EdgeGrad edge_words_rev(const Phys &p, bool wall, float nx, float ny,
         gcR += gSR0;
     }
     if (c_roe > 0.0f) {
-        const float t = gc_roe * 0.25f * p.g * rcp_of(p, c_roe);
+        const float t = gc_roe * 0.25f * p.g / c_roe;
         ghLs += t;
         ghRs += t;
     }
     if (roe_ok) {
-        const float per = gu_roe * rcp_of(p, den);
-        const float gsqL = per * (unL - u_roe), gsqR = per * (unR - u_roe);
-        gunL += per * sqL;
-        gunR += per * sqR;
-        // the roots' derivatives: 1 / (2 sqrt h), and root_g times it for the celerities
-        if (sqL > 0.0f) ghLs += (gsqL + gcL * root_g) * 0.5f * rcp_of(p, sqL);
-        if (sqR > 0.0f) ghRs += (gsqR + gcR * root_g) * 0.5f * rcp_of(p, sqR);
-    } else {
-        if (cL > 0.0f) ghLs += gcL * 0.5f * p.g / cL;
-        if (cR > 0.0f) ghRs += gcR * 0.5f * p.g / cR;
+        const float gsqL = gu_roe * (unL - u_roe) / den, gsqR = gu_roe * (unR - u_roe) / den;
+        gunL += gu_roe * sqL / den;
+        gunR += gu_roe * sqR / den;
+        if (sqL > 0.0f) ghLs += gsqL * 0.5f / sqL;
+        if (sqR > 0.0f) ghRs += gsqR * 0.5f / sqR;
     }
+    if (cL > 0.0f) ghLs += gcL * 0.5f * p.g / cL;
+    if (cR > 0.0f) ghRs += gcR * 0.5f * p.g / cR;
     // face-frame velocities
     float ghqnL = 0.0f, ghqtL = 0.0f, ghqnR = 0.0f, ghqtR = 0.0f;
     safe_vel_rev(p, hLs, hqnL, gunL, ghLs, ghqnL);
@@ -597,10 +587,10 @@ __global__ void __launch_bounds__(kThreads)
     adj_cell1(m, T, a, p, k, tag);
 }
 
-// The edge phases are bound by latency: a chain of loads (list, tile, records, states) and some 500 dependent
-// operations per tile. 64 registers let 592 CTAs be resident, one tile each at 250k cells with 14 % active (where
-// 100 registers took two rounds): edge<1>, with the predictor's cell update, 21.6 + 6.9 -> 14.2 us, edge<0>
-// 20.8 -> 9.7 us; the shared branch-free reciprocals are about half of the gain.
+// The edge phases are bound by latency: a chain of loads (list, tile, records, states), then some 25 IEEE quotients
+// in turn per edge (shared reciprocals would take 14 and 10 us instead of 21 and 16, but move the knots' float64
+// gradients by 1e-7). 64 registers let 592 CTAs be resident, one tile each at 250k cells with 14 % active, where
+// 100 registers took two rounds: edge<1> with the predictor's cell update 27.2 -> 21.3 us, edge<0> 20.9 -> 16.3 us.
 constexpr int kAdjEdgeCtas = 4;
 
 template <int STAGE>
