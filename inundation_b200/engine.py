@@ -22,7 +22,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import native
-from .layout import TileLayout, TileSet
+from .layout import NO_CELL, TileLayout, TileSet, halo_records
 from .sources import NO_HYDROGRAPH, Hydrograph
 from .tuning import ACTIVE_BLOCK_CELLS, B200_BACKEND, CFL_DEFAULT, DRY_TOL_DEFAULT, GRAVITY_G, OPEN_INFLOW, OPEN_STAGE
 
@@ -179,24 +179,26 @@ class ResidentEngine:
         self._blocks = None
         if not self._staged_fits or not self.packed_blocks:
             return
-        local = self._dev(_i32(B.local)).view(torch.float32)
+        H = halo_records(B, t["tile_cl"], t["tile_cr"], self.layout.n_padded_cells)
+        if B.tile_cells + H.max_halo >= NO_CELL:
+            return  # a local index has 16 bits
         self._blocks_t = {
-            "rec": torch.stack([t["tile_nx"], t["tile_ny"], t["tile_len"], local], dim=1),
+            "rec": torch.stack([t["tile_nx"], t["tile_ny"], t["tile_len"], H.local.view(torch.float32)], dim=1),
             "dz": torch.stack([t["tile_dzl"], t["tile_dzr"]], dim=1),
-            "halo": self._dev(B.halo), "halo_ptr": self._dev(_i32(B.halo_ptr)),
+            "halo": H.halo, "halo_ptr": H.halo_ptr,
         }
         dz = self._blocks_t["dz"]
         if not bool(((dz >= 0.0) & (dz <= 2.0**19)).all()):
             return  # not the face steps of a bed: the kernel's range check relies on them
         # every cell's perimeter, rounded up by more than the order of summing its edges can change
-        own = (local.view(torch.int32) & 0xFFFF) < B.tile_cells  # records in the tile of their left cell: each edge once
+        own = (H.local & 0xFFFF) < B.tile_cells  # records in the tile of their left cell: each edge once
         inner = own & (t["tile_cr"] >= 0)
         around = torch.zeros(self.layout.n_padded_cells, dtype=torch.float64, device=self.device)
         length = t["tile_len"].double()
         around.index_add_(0, t["tile_cl"], torch.where(own, length, 0.0))
         around.index_add_(0, t["tile_cr"].clamp(min=0), torch.where(inner, length, 0.0))
         self._blocks_t["perim"] = (around * (1.0 + 1e-4)).float()
-        blocks = native.SweBlocks(max_halo=B.max_halo, **{k: v.data_ptr() for k, v in self._blocks_t.items()})
+        blocks = native.SweBlocks(max_halo=H.max_halo, **{k: v.data_ptr() for k, v in self._blocks_t.items()})
         per_sm = ctypes.c_int(0)
         with torch.cuda.device(self.device):
             native.check(self._lib.swe_configure_blocks(ctypes.byref(self._mesh), ctypes.byref(blocks),

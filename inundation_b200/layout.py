@@ -34,6 +34,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 
 import numpy as np
+import torch
 from numpy.typing import NDArray
 
 from .mesh.blocks import block_adjacency, block_two_ring, edge_order_by_block, remap_cell_edges
@@ -67,16 +68,6 @@ class TileSet:
     lcsr: NDArray[np.uint16]  # per CSR slot, flat in global slot order
     lcsr_blk: NDArray[np.uint16]  # the same, regrouped per tile from lcsr_ptr[t]
     lcsr_ptr: NDArray[np.uint32]  # n_tiles + 1, multiples of 8 (16-byte aligned segments)
-    # The cells a tile's records read outside it, each once, by cell id, and every record's two cells as
-    # tile-local indices, left | right << 16: a cell of the tile by its place in it, the k-th halo cell as
-    # tile_cells + k, NO_CELL beyond a boundary edge.
-    halo: NDArray[np.int32] | None = None
-    halo_ptr: NDArray[np.uint32] | None = None  # n_tiles + 1
-    local: NDArray[np.uint32] | None = None
-
-    @property
-    def max_halo(self) -> int:
-        return 0 if self.halo_ptr is None else int(np.diff(self.halo_ptr.astype(np.int64)).max())
 
 
 @dataclass
@@ -201,31 +192,46 @@ def _tile_set(geom: MeshGeometry, order: NDArray[np.int64], signed: NDArray[np.i
     )
 
 
-def _add_halo(T: TileSet, n_cells: int) -> None:
-    """The halo lists and local record indices of a tile set (see ``TileSet``)."""
-    size = T.tile_cells
-    tile = np.repeat(np.arange(T.n_tiles, dtype=np.int64), np.diff(T.ptr.astype(np.int64)))
-    base = tile * size
-    cl, cr = T.cl.astype(np.int64), T.cr.astype(np.int64)
-    real = T.edge >= 0
-    out_l = real & ((cl < base) | (cl >= base + size))
-    out_r = real & (cr >= 0) & ((cr < base) | (cr >= base + size))
-    at_l, at_r = np.flatnonzero(out_l), np.flatnonzero(out_r)
-    key = np.concatenate([tile[at_l] * n_cells + cl[at_l], tile[at_r] * n_cells + cr[at_r]])
-    unique, place = np.unique(key, return_inverse=True)
+@dataclass
+class HaloRecords:
+    """The cells that each tile's records read outside it, each once, by cell id, and every record's two
+    cells as tile-local indices: a cell of the tile by its place in it, the k-th halo cell as ``tile_cells + k``,
+    ``NO_CELL`` beyond a boundary edge (and 0 in padding)."""
+
+    halo: torch.Tensor  # int32
+    halo_ptr: torch.Tensor  # int32, n_tiles + 1
+    local: torch.Tensor  # int32: left | right << 16
+    max_halo: int
+
+
+def halo_records(T: TileSet, cl: torch.Tensor, cr: torch.Tensor, n_cells: int) -> HaloRecords:
+    """Halo lists and local indices of a tile set, on the device of its records' cells ``cl`` and ``cr``
+    (a sort of the records that leave their tile; on the GPU a few ms for a million cells)."""
+    dev, size = cl.device, T.tile_cells
+    ptr = torch.from_numpy(T.ptr.astype(np.int64)).to(dev)
+    count = torch.from_numpy(T.count.astype(np.int64)).to(dev)
+    tile = torch.repeat_interleave(torch.arange(T.n_tiles, device=dev), ptr.diff(), output_size=cl.numel())
+    real = torch.arange(cl.numel(), device=dev) - ptr[tile] < count[tile]
+    left, right = cl.long() - tile * size, cr.long() - tile * size
+    boundary = cr < 0
+    at_l = torch.nonzero(real & ((left < 0) | (left >= size))).flatten()
+    at_r = torch.nonzero(real & ~boundary & ((right < 0) | (right >= size))).flatten()
+    key = torch.cat([tile[at_l] * n_cells + cl[at_l], tile[at_r] * n_cells + cr[at_r]])
+    unique, place = torch.unique(key, return_inverse=True)
     owner = unique // n_cells
-    ptr = np.searchsorted(owner, np.arange(T.n_tiles + 1))
-    T.halo = (unique - owner * n_cells).astype(np.int32) if unique.size else np.zeros(1, np.int32)
-    T.halo_ptr = ptr.astype(np.uint32)
-    if size + T.max_halo >= NO_CELL:
-        raise ValueError(f"a tile reads {T.max_halo} cells outside it; the limit is {NO_CELL - size - 1}")
-    slot = size + place - ptr[owner[place]]
-    left, right = cl - base, cr - base
-    left[at_l] = slot[: at_l.size]
-    right[at_r] = slot[at_l.size :]
-    right[cr < 0] = NO_CELL
-    left[~real] = right[~real] = 0
-    T.local = (left | (right << 16)).astype(np.uint32)
+    halo_ptr = torch.searchsorted(owner, torch.arange(T.n_tiles + 1, device=dev))
+    slot = size + place - halo_ptr[owner[place]]
+    left[at_l] = slot[: at_l.numel()]
+    right[at_r] = slot[at_l.numel() :]
+    right[boundary] = NO_CELL
+    local = torch.where(real, left | (right << 16), 0)
+    halo = (unique - owner * n_cells).int()
+    return HaloRecords(
+        halo=halo if halo.numel() else torch.zeros(1, dtype=torch.int32, device=dev),
+        halo_ptr=halo_ptr.int(),
+        local=torch.where(local >= 1 << 31, local - (1 << 32), local).int(),
+        max_halo=int(halo_ptr.diff().max()),
+    )
 
 
 def build_tile_layout(geom: MeshGeometry) -> TileLayout:
@@ -258,14 +264,12 @@ def _build(geom) -> TileLayout:
     ecl = geom.edge_cellL[order].astype(np.int32)
     ecr = geom.edge_cellR[order].astype(np.int32)
     rptr, ridx = block_two_ring(*block_adjacency(ecl, ecr, n, bc))
-    blocks = _tile_set(geom, order, signed, bc)
-    _add_halo(blocks, n)
     return TileLayout(
         n_cells=n,
         n_edges=n_e,
         n_blocks=n_blk,
         edge_order=order,
-        blocks=blocks,
+        blocks=_tile_set(geom, order, signed, bc),
         subs=_tile_set(geom, order, signed, SUB_TILE_CELLS),
         cptr=cptr_pad.astype(np.uint32),
         ring_ptr=rptr.astype(np.uint32),

@@ -4,8 +4,9 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+import torch
 
-from inundation_b200.layout import NO_CELL, build_batch_layout, build_tile_layout
+from inundation_b200.layout import NO_CELL, build_batch_layout, build_tile_layout, halo_records
 from inundation_b200.scenarios import open_channel, voronoi_geometry
 
 
@@ -18,19 +19,22 @@ def test_local_indices_name_the_records_cells(cells: int) -> None:
     else:
         layout = build_tile_layout(voronoi_geometry(cells, 10.0 * cells**0.5, cells))
     T = layout.blocks
+    H = halo_records(T, torch.from_numpy(T.cl), torch.from_numpy(T.cr), layout.n_padded_cells)
+    halo, halo_ptr = H.halo.numpy(), H.halo_ptr.numpy().astype(np.int64)
+    local = H.local.numpy().view(np.uint32)
     tile = np.repeat(np.arange(T.n_tiles), np.diff(T.ptr.astype(np.int64)))
     real = T.edge >= 0
 
-    def cell(local: np.ndarray) -> np.ndarray:
-        place = T.halo_ptr[tile].astype(np.int64) + np.maximum(local.astype(np.int64) - 256, 0)
-        return np.where(local < 256, 256 * tile + local, T.halo[np.minimum(place, T.halo.size - 1)])
+    def cell(index: np.ndarray) -> np.ndarray:
+        place = halo_ptr[tile] + np.maximum(index.astype(np.int64) - 256, 0)
+        return np.where(index < 256, 256 * tile + index, halo[np.minimum(place, halo.size - 1)])
 
-    left, right = T.local & 0xFFFF, T.local >> 16
+    left, right = local & 0xFFFF, local >> 16
     np.testing.assert_array_equal(cell(left)[real], T.cl[real])
     inner = real & (T.cr >= 0)
     np.testing.assert_array_equal(cell(right)[inner], T.cr[inner])
     assert (right[real & (T.cr < 0)] == NO_CELL).all() and (left[real & (T.cr < 0)] < 256).all()
     for t in range(T.n_tiles):  # each cell outside once
-        halo = T.halo[int(T.halo_ptr[t]) : int(T.halo_ptr[t + 1])]
-        assert np.unique(halo).size == halo.size and not ((halo // 256) == t).any()
-    assert T.max_halo == int(np.diff(T.halo_ptr.astype(np.int64)).max(initial=0))
+        own = halo[halo_ptr[t] : halo_ptr[t + 1]]
+        assert np.unique(own).size == own.size and not ((own // 256) == t).any()
+    assert H.max_halo == int(np.diff(halo_ptr).max(initial=0))
