@@ -348,6 +348,13 @@ int swe_tape_record(const swe_mesh_t *mesh, const swe_state_t *state, const swe_
    control block's count of real steps); record == 0 adds the squared misfit against that row to *loss. */
 int swe_gauge_misfit(const swe_state_t *state, const swe_gauges_t *gauges, int record, swe_stream_t stream);
 
+/* n_steps whole steps of kernel 2 (swe_steps) with swe_gauge_misfit after each, in the one persistent
+   launch; single-instance closed meshes, compensated, without the clamp diagnostic. The gauges' rows
+   follow the control block's count of steps at the launch. */
+int swe_steps_gauged(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
+                     const swe_sources_t *sources, const swe_gauges_t *gauges, int record, uint32_t n_steps,
+                     swe_stream_t stream);
+
 /* Reverses tape slots `slots - 1` down to 0 (slot k is the step from tape state k to k + 1):
    for each, adds the misfit's gradient at the state after the step (obs row row0 + k), then
    takes the adjoint back through the sources, the corrector and the predictor, accumulating

@@ -31,7 +31,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import native
-from .engine import ResidentEngine, START
+from .engine import AUTO_DENSE_FRACTION, KERNELS, START, ResidentEngine
 from .layout import build_tile_layout
 from .mesh.geometry import MeshGeometry
 from .sources import Hydrograph
@@ -63,6 +63,9 @@ class GaugeCalibration(ResidentEngine):
     # the segment graphs capture one swe_step per step: a per-step stage kernel
     stage_kernel: str = "tiled"
     packed_blocks: bool = False  # every step is one swe_step, and set_parameters moves the bed steps
+    # run the forward in the persistent kernel, gauges included, while few blocks are active (as "auto"
+    # does); False, more blocks, or another stage kernel: graphs of the per-step kernels. The same bits.
+    persistent_forward: bool = True
     # reverse each segment in one cooperative launch (grid barriers between phases) instead of one
     # launch per phase and step; the arithmetic is the same. Off by default: at 250k cells the
     # per-phase launches fill more SMs and measured faster (121 against 135 ms for 2000 steps).
@@ -175,7 +178,7 @@ class GaugeCalibration(ResidentEngine):
     def _state_tensors(self) -> dict[str, torch.Tensor]:
         d = {name: self._t[name] for name in _SNAPSHOT}
         d.update(blk=self._blk, active_list=self._active_list, items=self._items, sched=self._sched,
-                 dt_buf=self._dt_buf, ctrl=self._ctrl_dev)
+                 marks=self._marks, dt_buf=self._dt_buf, ctrl=self._ctrl_dev)
         return d
 
     def _snapshot_into(self, idx: int) -> None:
@@ -228,6 +231,25 @@ class GaugeCalibration(ResidentEngine):
             self._segment_graphs[key] = graph
         return graph
 
+    def _forward_steps(self, n_steps: int, record: int) -> None:
+        """``n_steps`` steps with the gauges after each, on the solver's stream."""
+        grid = self.grid(KERNELS["persistent"])
+        sparse = self._active_blocks <= AUTO_DENSE_FRACTION * self.n_blocks or 4 * self._active_blocks <= grid
+        if self.persistent_forward and self.stage_kernel == "tiled" and not self.track_clamp and self._persistent_fits \
+                and sparse:
+            params, sources = self._params(), self._sources()
+            params.kernel, params.grid = KERNELS["persistent"], grid
+            native.check(
+                self._lib.swe_steps_gauged(ctypes.byref(self._mesh), ctypes.byref(self._state), ctypes.byref(params),
+                                           ctypes.byref(sources), ctypes.byref(self._gauges), record, n_steps,
+                                           self._cuda_stream),
+                "swe_steps_gauged",
+            )
+            return
+        graph = self._segment_graph(n_steps, record)
+        with torch.cuda.stream(self._stream):
+            graph.replay()
+
     def _taped_graph(self, n_steps: int) -> torch.cuda.CUDAGraph:
         key = ("tape", n_steps, self._src_version)
         graph = self._segment_graphs.get(key)
@@ -259,15 +281,15 @@ class GaugeCalibration(ResidentEngine):
         if not self.compensated:
             raise ValueError("the adjoint differentiates the compensated step; keep compensated=True")
         self._start()
+        if self.persistent_forward:
+            self._read_ctrl()  # the active blocks of the initial state choose the forward's kernel
         done = 0
         seg = 0
         while done < self.steps:
             n = min(self.K, self.steps - done)
             if checkpoints:
                 self._snapshot_into(seg)
-            graph = self._segment_graph(n, record)
-            with torch.cuda.stream(self._stream):
-                graph.replay()
+            self._forward_steps(n, record)
             done += n
             seg += 1
         self._read_ctrl()

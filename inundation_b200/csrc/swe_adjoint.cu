@@ -28,6 +28,7 @@
 
 #include <cstdint>
 
+#include "swe_gauges.cuh"
 #include "swe_grid.cuh"
 
 namespace swe {
@@ -654,29 +655,7 @@ __global__ void tape_record_kernel(swe_mesh_t m, swe_state_t s, swe_tape_t T, ui
 // Gauge record (record = 1) or misfit accumulation, after a step.
 __global__ void __launch_bounds__(kThreads) gauge_kernel(swe_state_t s, swe_gauges_t gg, int record) {
     __shared__ double acc[kThreads];
-    const uint64_t done = s.ctrl->steps;
-    double sum = 0.0;
-    if (done >= 1 && done <= gg.steps) {
-        float *row = gg.obs + static_cast<size_t>(done - 1) * gg.count;
-        for (uint32_t g = threadIdx.x; g < gg.count; g += kThreads) {
-            const uint32_t c = gg.cells[g];
-            const float H = s.h[c] + s.h_lo[c];
-            if (record) {
-                row[g] = H;
-            } else {
-                const double d = static_cast<double>(H) - static_cast<double>(row[g]);
-                sum += d * d;
-            }
-        }
-    }
-    if (record) return;
-    acc[threadIdx.x] = sum;
-    __syncthreads();
-    for (int w = kThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) acc[threadIdx.x] += acc[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *gg.loss += acc[0];
+    gauge_after_step(s, gg, record, s.ctrl->steps, acc);
 }
 
 __global__ void bed_steps_kernel(const int32_t *cl, const int32_t *cr, const float *z, float *dzl, float *dzr,

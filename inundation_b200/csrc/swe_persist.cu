@@ -15,6 +15,7 @@
 
 #include <cstdint>
 
+#include "swe_gauges.cuh"
 #include "swe_grid.cuh"
 #include "swe_sources.cuh"
 #include "swe_tiled.cuh"
@@ -570,15 +571,19 @@ __device__ __forceinline__ void seat_handover(const swe_mesh_t &m, const swe_sta
     }
 }
 
-template <bool COMP, bool CLAMP, bool OPEN>
+// GAUGED: after every step the last CTA, which is the least likely to have a seat, reads the gauges (the state stands
+// still until the next corrector).
+template <bool COMP, bool CLAMP, bool OPEN, bool GAUGED = false>
 __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
     persistent_steps_kernel(swe_mesh_t m, swe_state_t s, swe_sources_t src, Phys p, float cfl, int all_active,
-                            uint32_t n_steps) {
+                            uint32_t n_steps, swe_gauges_t gauges, int record) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ TiledShared<kPersistThreads> sh;
     __shared__ SeatShared ss;
     __shared__ int flag[3];
     __shared__ uint32_t epoch0;
+    __shared__ double acc[GAUGED ? kPersistThreads : 1];
+    __shared__ uint64_t steps0;
     CountSync g{s.sync, 0u};  // the launch zeroes the counter before the kernel starts
     if (threadIdx.x == 0) {
         mbar_init(reinterpret_cast<uint64_t *>(smem), 1u);
@@ -588,6 +593,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         ss.seat = ss.staged = ss.kept = ss.kept_ring_block = kNoTile;
         ss.kept_bits_step = 0u;
         ss.state_ok = 0u;
+        if (GAUGED) steps0 = s.ctrl->steps;
         if (blockIdx.x == 0) {  // the queues of this launch start empty (first used after the first barrier)
             for (int k = 0; k < 2; ++k) {
                 s.sched[kSchedQProd + k] = 0u;
@@ -682,6 +688,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         // small mesh (8 fixed steps of 2048 cells took 1.02 ms of a 200-step launch). The control of the step
         // before wrote the word, so every CTA finds it here; read earlier, it would delay every corrector.
         if ((idle = static_cast<uint32_t>(flag[2]) == epoch)) break;
+        if (GAUGED && blockIdx.x == gridDim.x - 1u) gauge_after_step(s, gauges, record, steps0 + step + 1u, acc);
         // the hand-over reads the last step's dt and the lists its control zeroes
         if (last_step && !(ok = count_sync(g, flag, nothing))) break;
     }
@@ -692,10 +699,10 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
     }
 }
 
-template <bool COMP, bool CLAMP, bool OPEN>
+template <bool COMP, bool CLAMP, bool OPEN, bool GAUGED = false>
 int launch_persistent(const swe_mesh_t *m, const swe_state_t *s, const swe_params_t *p, const swe_sources_t *src,
-                      uint32_t n_steps, cudaStream_t st) {
-    auto kern = persistent_steps_kernel<COMP, CLAMP, OPEN>;
+                      uint32_t n_steps, cudaStream_t st, const swe_gauges_t *gauges = nullptr, int record = 0) {
+    auto kern = persistent_steps_kernel<COMP, CLAMP, OPEN, GAUGED>;
     const size_t bytes = tiled_smem_bytes(m->max_sub_edges, m->max_sub_slots, true);
     int rc = set_smem(kern, bytes);
     if (rc) return rc;
@@ -717,7 +724,9 @@ int launch_persistent(const swe_mesh_t *m, const swe_state_t *s, const swe_param
     swe_mesh_t mm = *m;
     swe_state_t ss = *s;
     swe_sources_t sc = *src;
-    void *args[] = {&mm, &ss, &sc, &ph, &cfl, &all_active, &n_steps};
+    swe_gauges_t gg{};
+    if (gauges) gg = *gauges;
+    void *args[] = {&mm, &ss, &sc, &ph, &cfl, &all_active, &n_steps, &gg, &record};
     // the grid barrier's arrival counter starts from zero in every launch
     if (cudaMemsetAsync(s->sync, 0, sizeof(uint32_t), st) != cudaSuccess) return SWE_ERR_CUDA;
     if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(grid), dim3(kPersistThreads), args, bytes,
@@ -756,6 +765,20 @@ int configure_persistent(const swe_mesh_t *mesh, int *blocks_per_sm) {
 }  // namespace swe
 
 using namespace swe;
+
+extern "C" int swe_steps_gauged(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
+                                const swe_sources_t *sources, const swe_gauges_t *gauges, int record, uint32_t n_steps,
+                                swe_stream_t stream) {
+    if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources || !gauges || mesh->n_open || mesh->n_inst != 1u ||
+        !params->compensated || params->track_clamp)
+        return SWE_ERR_ARGUMENT;
+    if (!gauges->cells || !gauges->obs || (!record && !gauges->loss) || gauges->count == 0u) return SWE_ERR_ARGUMENT;
+    if (!state->sync || !state->marks || (reinterpret_cast<uintptr_t>(state->dt_buf) & 15u)) return SWE_ERR_ARGUMENT;
+    if (mesh->max_sub_edges > 2047u || mesh->max_sub_slots > 2047u) return SWE_ERR_TOO_LARGE;
+    if (sources->count && (!sources->cells || !sources->rate)) return SWE_ERR_ARGUMENT;
+    if (n_steps == 0u) return SWE_OK;
+    return launch_persistent<true, false, false, true>(mesh, state, params, sources, n_steps, stream, gauges, record);
+}
 
 extern "C" int swe_steps(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
                          const swe_sources_t *sources, uint32_t n_steps, swe_stream_t stream) {

@@ -50,6 +50,7 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "swe_stage_taped": ([_P, _P, _P, ctypes.c_int, _P, _P], ctypes.c_int),
     "swe_tape_record": ([_P, _P, _P, _U32, _P], ctypes.c_int),
     "swe_gauge_misfit": ([_P, _P, ctypes.c_int, _P], ctypes.c_int),
+    "swe_steps_gauged": ([_P, _P, _P, _P, _P, ctypes.c_int, _U32, _P], ctypes.c_int),
     "swe_adjoint_segment": ([_P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _P], ctypes.c_int),
 }
 
