@@ -220,8 +220,7 @@ class GaugeCalibration(ResidentEngine):
             params, sources = self._params(), self._sources()
             mesh, state = ctypes.byref(self._mesh), ctypes.byref(self._state)
             graph = torch.cuda.CUDAGraph()
-            self._stream.synchronize()
-            with torch.cuda.graph(graph, stream=self._stream):
+            with self._capture(graph):
                 st = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
                 for _ in range(n_steps):
                     native.check(self._lib.swe_step(mesh, state, ctypes.byref(params), ctypes.byref(sources), st),
@@ -260,8 +259,7 @@ class GaugeCalibration(ResidentEngine):
             n = self.layout.n_padded_cells
             s0, s1 = self._tape_t["s0"], self._tape_t["s1"]
             graph = torch.cuda.CUDAGraph()
-            self._stream.synchronize()
-            with torch.cuda.graph(graph, stream=self._stream):
+            with self._capture(graph):
                 st = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
                 pp, sp = ctypes.byref(params), ctypes.byref(sources)
                 for j in range(n_steps):
