@@ -481,7 +481,8 @@ def forward_line(args, sc, world: int, local: int):
             "frac": achieved / peak,
             "traffic": traffic,
             "kernel": f"stage kernel, {args.kernel} (fused edge flux + gather + Heun update), both stages"
-            if events else "persistent step kernel (whole steps: both stages, dilation, step control; grid barriers)",
+            if events else f"{'persistent' if args.kernel == 'persistent' else 'dense'} step kernel (whole steps: both "
+            "stages, dilation, step control; grid barriers)",
             "algorithmic_bytes_per_cell_step": bpc,
             "launches": launches,
             "mean_launch_us": stage_ms * 1e3 / launches,
