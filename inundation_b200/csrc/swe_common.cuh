@@ -282,6 +282,14 @@ inline bool mesh_ok(const swe_mesh_t *m) {
 // The open-edge tally words must exist when the mesh has open edges.
 inline bool open_ok(const swe_mesh_t *m, const swe_state_t *s) { return m->n_open == 0u || s->open_vol; }
 
+// Sources need their cells and rates, hydrographs their knots.
+inline bool sources_ok(const swe_sources_t *s) {
+    if (!s) return false;
+    if (s->count == 0u) return true;
+    if (!s->cells || !s->rate) return false;
+    return !s->hydro || (s->hscale && s->knot_ptr && s->knot_t && s->knot_q && s->n_hydro);
+}
+
 inline bool state_ok(const swe_state_t *s) {
     return s && s->h && s->hu && s->hv && s->h_lo && s->h1 && s->hu1 && s->hv1 && s->h1_lo && s->clamp_mass &&
            s->blk && s->active_list && s->items && s->sched && s->dt_buf && s->ctrl;

@@ -241,12 +241,8 @@ size_t swe_workspace_bytes(uint32_t n_blocks, uint32_t n_inst) {
 
 int swe_apply_sources(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
                       const swe_sources_t *sources, swe_stream_t stream) {
-    if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources) return SWE_ERR_ARGUMENT;
+    if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources_ok(sources)) return SWE_ERR_ARGUMENT;
     if (sources->count == 0u) return SWE_OK;
-    if (!sources->cells || !sources->rate) return SWE_ERR_ARGUMENT;
-    if (sources->hydro &&
-        (!sources->hscale || !sources->knot_ptr || !sources->knot_t || !sources->knot_q || sources->n_hydro == 0u))
-        return SWE_ERR_ARGUMENT;
     // One launch instead of two up to a CTA's worth of sources, 8 lanes each for the bounds (one source: 4.2 us
     // against 3.2 + 4.5); more take the passes, whose threads spread over the GPU.
     if (sources->count <= kThreads) {

@@ -424,13 +424,11 @@ int swe_configure_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, int
 
 int swe_steps_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, const swe_state_t *state,
                      const swe_params_t *params, const swe_sources_t *sources, uint32_t n_steps, swe_stream_t stream) {
-    if (!mesh_ok(mesh) || !blocks_ok(mesh, blocks) || !state_ok(state) || !open_ok(mesh, state) || !params || !sources)
+    if (!mesh_ok(mesh) || !blocks_ok(mesh, blocks) || !state_ok(state) || !open_ok(mesh, state) || !params ||
+        !sources_ok(sources))
         return SWE_ERR_ARGUMENT;
     if (!state->sync || (reinterpret_cast<uintptr_t>(state->dt_buf) & 15u)) return SWE_ERR_ARGUMENT;
-    if (sources->count && (!sources->cells || !sources->rate || !blocks->src_ptr)) return SWE_ERR_ARGUMENT;
-    if (sources->count && sources->hydro &&
-        (!sources->hscale || !sources->knot_ptr || !sources->knot_t || !sources->knot_q || sources->n_hydro == 0u))
-        return SWE_ERR_ARGUMENT;
+    if (sources->count && !blocks->src_ptr) return SWE_ERR_ARGUMENT;
     if (mesh->max_sub_edges > 2047u || mesh->max_sub_slots > 2047u || mesh->n_inst > 1023u ||
         mesh->n_blocks > (1u << 23) || kBlockCells + blocks->max_halo >= kNoCell ||
         mesh->max_tile_edges > 32u * kThreads)

@@ -769,13 +769,12 @@ using namespace swe;
 extern "C" int swe_steps_gauged(const swe_mesh_t *mesh, const swe_state_t *state, const swe_params_t *params,
                                 const swe_sources_t *sources, const swe_gauges_t *gauges, int record, uint32_t n_steps,
                                 swe_stream_t stream) {
-    if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources || !gauges || mesh->n_open || mesh->n_inst != 1u ||
-        !params->compensated || params->track_clamp)
+    if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources_ok(sources) || !gauges || mesh->n_open ||
+        mesh->n_inst != 1u || !params->compensated || params->track_clamp)
         return SWE_ERR_ARGUMENT;
     if (!gauges->cells || !gauges->obs || (!record && !gauges->loss) || gauges->count == 0u) return SWE_ERR_ARGUMENT;
     if (!state->sync || !state->marks || (reinterpret_cast<uintptr_t>(state->dt_buf) & 15u)) return SWE_ERR_ARGUMENT;
     if (mesh->max_sub_edges > 2047u || mesh->max_sub_slots > 2047u) return SWE_ERR_TOO_LARGE;
-    if (sources->count && (!sources->cells || !sources->rate)) return SWE_ERR_ARGUMENT;
     if (n_steps == 0u) return SWE_OK;
     return launch_persistent<true, false, false, true>(mesh, state, params, sources, n_steps, stream, gauges, record);
 }
@@ -794,7 +793,7 @@ extern "C" int swe_steps(const swe_mesh_t *mesh, const swe_state_t *state, const
     }
     if (!state->sync || !state->marks || (reinterpret_cast<uintptr_t>(state->dt_buf) & 15u)) return SWE_ERR_ARGUMENT;
     if (mesh->max_sub_edges > 2047u || mesh->max_sub_slots > 2047u || mesh->n_inst > 1023u) return SWE_ERR_TOO_LARGE;
-    if (sources->count && (!sources->cells || !sources->rate)) return SWE_ERR_ARGUMENT;
+    if (!sources_ok(sources)) return SWE_ERR_ARGUMENT;
     return mesh->n_open ? dispatch_persistent<true>(mesh, state, params, sources, n_steps, stream)
                         : dispatch_persistent<false>(mesh, state, params, sources, n_steps, stream);
 }

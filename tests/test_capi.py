@@ -169,3 +169,91 @@ def test_the_dt_wait_probe_refuses_a_misaligned_or_missing_buffer(lib: ctypes.CD
     assert lib.swe_dt_wait_probe(ctypes.byref(state), 1, ctypes.c_void_p(16), None) == 1  # no dt words
     state.dt_buf, state.ctrl = 0x20008, 0x30000
     assert lib.swe_dt_wait_probe(ctypes.byref(state), 1, ctypes.c_void_p(16), None) == 1  # not 16-byte aligned
+
+
+def _placeholders(**mesh_fields):
+    """Structs with placeholder addresses that nothing dereferences: the argument checks run on the host."""
+    mesh = native.SweMesh(n_cells=256, n_blocks=1, max_tile_edges=64, n_inst=1, max_sub_edges=64, max_sub_slots=64)
+    for name, kind in native.SweMesh._fields_:
+        if kind is native._P and name != "open_cond":
+            setattr(mesh, name, 0x10000)
+    for name, value in mesh_fields.items():
+        setattr(mesh, name, value)
+    blocks = native.SweBlocks(max_halo=64, **{name: 0x30000 for name, kind in native.SweBlocks._fields_ if kind is native._P})
+    state = native.SweState(**{name: 0x20000 for name, _ in native.SweState._fields_})
+    params = native.SweParams(g=9.81, dry_tol=1e-4, cfl=0.8, compensated=1, active_set=1, kernel=2)
+    gauges = native.SweGauges(cells=0x40000, obs=0x40000, loss=0x40000, count=1, steps=1)
+    return mesh, blocks, state, params, gauges
+
+
+@pytest.mark.parametrize("missing", ["hscale", "knot_ptr", "knot_t", "knot_q", "n_hydro"])
+@pytest.mark.parametrize("entry", ["swe_steps", "swe_steps_gauged", "swe_steps_blocks"])
+def test_whole_steps_refuse_hydrographs_without_their_knots(lib: ctypes.CDLL, entry: str, missing: str) -> None:
+    mesh, blocks, state, params, gauges = (ctypes.byref(s) for s in _placeholders())
+    sources = native.SweSources(cells=0x50000, rate=0x50000, hydro=0x50000, hscale=0x50000, knot_ptr=0x50000, knot_t=0x50000,
+                                knot_q=0x50000, count=1, n_hydro=1)
+    setattr(sources, missing, 0 if missing == "n_hydro" else None)
+    src = ctypes.byref(sources)
+    rc = {"swe_steps": lambda: lib.swe_steps(mesh, state, params, src, 1, None),
+          "swe_steps_gauged": lambda: lib.swe_steps_gauged(mesh, state, params, src, gauges, 0, 1, None),
+          "swe_steps_blocks": lambda: lib.swe_steps_blocks(mesh, blocks, state, params, src, 1, None)}[entry]()
+    assert rc == 1
+
+
+def test_block_steps_refuse_missing_records_and_sizes(lib: ctypes.CDLL) -> None:
+    sources = native.SweSources()
+    for name, kind in native.SweBlocks._fields_:
+        if kind is native._P and name != "src_ptr":  # src_ptr: only with sources
+            mesh, blocks, state, params, _ = _placeholders()
+            setattr(blocks, name, None)
+            per_sm = ctypes.c_int(7)
+            assert lib.swe_steps_blocks(*map(ctypes.byref, (mesh, blocks, state, params, sources)), 1, None) == 1
+            assert lib.swe_configure_blocks(ctypes.byref(mesh), ctypes.byref(blocks), ctypes.byref(per_sm)) == 1
+    mesh, blocks, state, params, _ = _placeholders()
+    with_sources = native.SweSources(cells=0x50000, rate=0x50000, count=1)
+    blocks.src_ptr = None
+    assert lib.swe_steps_blocks(*map(ctypes.byref, (mesh, blocks, state, params, with_sources)), 1, None) == 1
+    for change in ({"sync": None}, {"dt_buf": 0x20008}, {"h1": None}):
+        mesh, blocks, state, params, _ = _placeholders()
+        for name, value in change.items():
+            setattr(state, name, value)
+        assert lib.swe_steps_blocks(*map(ctypes.byref, (mesh, blocks, state, params, sources)), 1, None) == 1
+    for change in ({"max_sub_edges": 2048}, {"max_sub_slots": 2048}, {"n_inst": 1024}, {"n_blocks": (1 << 23) + 1},
+                   {"max_tile_edges": 32 * 256 + 1}):
+        mesh, blocks, state, params, _ = _placeholders(**change)
+        assert lib.swe_steps_blocks(*map(ctypes.byref, (mesh, blocks, state, params, sources)), 1, None) == 3
+    mesh, blocks, state, params, _ = _placeholders()
+    blocks.max_halo = 0xFFFF - 256
+    assert lib.swe_steps_blocks(*map(ctypes.byref, (mesh, blocks, state, params, sources)), 1, None) == 3
+    per_sm = ctypes.c_int(7)
+    assert lib.swe_configure_blocks(ctypes.byref(mesh), ctypes.byref(blocks), ctypes.byref(per_sm)) == 0
+    assert per_sm.value == 0  # does not fit: no error
+
+
+def test_gauged_steps_refuse_what_they_do_not_run(lib: ctypes.CDLL) -> None:
+    sources = native.SweSources()
+
+    def rc(mesh, state, params, gauges, record: int = 0) -> int:
+        return lib.swe_steps_gauged(*map(ctypes.byref, (mesh, state, params, sources, gauges)), record, 1, None)
+
+    for change in ({"n_open": 1, "open_cond": 0x10000}, {"n_inst": 2}, {"area": None}):
+        mesh, _, state, params, gauges = _placeholders(**change)
+        assert rc(mesh, state, params, gauges) == 1
+    for change in ({"compensated": 0}, {"track_clamp": 1}):
+        mesh, _, state, params, gauges = _placeholders()
+        for name, value in change.items():
+            setattr(params, name, value)
+        assert rc(mesh, state, params, gauges) == 1
+    for change in ({"cells": None}, {"obs": None}, {"loss": None}, {"count": 0}):
+        mesh, _, state, params, gauges = _placeholders()
+        for name, value in change.items():
+            setattr(gauges, name, value)
+        assert rc(mesh, state, params, gauges) == 1
+    for change in ({"sync": None}, {"marks": None}, {"dt_buf": 0x20008}):
+        mesh, _, state, params, gauges = _placeholders()
+        for name, value in change.items():
+            setattr(state, name, value)
+        assert rc(mesh, state, params, gauges) == 1
+    for change in ({"max_sub_edges": 2048}, {"max_sub_slots": 2048}):
+        mesh, _, state, params, gauges = _placeholders(**change)
+        assert rc(mesh, state, params, gauges) == 3
