@@ -209,6 +209,8 @@ int launch_handover(const swe_mesh_t *m, const swe_state_t *s, const swe_params_
     return check_launch();
 }
 
+constexpr uint32_t kFewSources = 128;
+
 // A few sources in one CTA: the increments, then the bounds, without a launch between them.
 __global__ void __launch_bounds__(kThreads)
     source_few_kernel(swe_mesh_t m, swe_state_t s, swe_sources_t src, Phys p, float cfl, int comp) {
@@ -243,9 +245,10 @@ int swe_apply_sources(const swe_mesh_t *mesh, const swe_state_t *state, const sw
                       const swe_sources_t *sources, swe_stream_t stream) {
     if (!mesh_ok(mesh) || !state_ok(state) || !params || !sources_ok(sources)) return SWE_ERR_ARGUMENT;
     if (sources->count == 0u) return SWE_OK;
-    // One launch instead of two up to a CTA's worth of sources, 8 lanes each for the bounds (one source: 4.2 us
-    // against 3.2 + 4.5); more take the passes, whose threads spread over the GPU.
-    if (sources->count <= kThreads) {
+    // One launch instead of two for a few sources, 8 lanes each for the bounds (one source: 4.2 us against 3.2 + 4.5).
+    // The CTA takes 32 bounds in a round of 3 us, so more go to the passes, whose threads spread over the GPU: a step of
+    // 30k cells takes 29.0 us with 64 sources in one CTA and 33.3 in two passes, with 128 32.9 and 33.5, with 256 38.0 and 33.1.
+    if (sources->count <= kFewSources) {
         source_few_kernel<<<1, kThreads, 0, stream>>>(*mesh, *state, *sources, make_phys(params->g, params->dry_tol),
                                                       params->cfl, static_cast<int>(params->compensated));
         return check_launch();

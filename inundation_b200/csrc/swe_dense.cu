@@ -15,8 +15,8 @@
 // counter, so that the active blocks spread evenly over the SMs, wherever they lie, and every
 // CTA ends within about a block of the others; its corrector repeats the blocks it took.
 // Sources come by block: a block's are added right after its corrector's update. Those of
-// inactive blocks wait for one more barrier, in the steps that have any. The CFL bounds of a few
-// sources are taken by the step control's CTA; those of many (rain) by a pass over all of them
+// inactive blocks wait for one more barrier, in the steps that have any. The CFL bounds of up
+// to kCtaBounds sources are taken by the step control's CTA; those of more by a pass over all of them
 // after a barrier, which looks only at the cells whose bound can be below the smallest one so far:
 // a source's wave speeds are at most u + 2c on its whole perimeter.
 // Bound: instruction issue (a steady 75-80 % of the slots; DRAM and L2 stay below 20 % of their peaks), then a
@@ -315,12 +315,12 @@ __global__ void __launch_bounds__(kThreads, kDenseMinCtas)
                         s.blk[kBlkWords * b + kBlkWet] = 1u;
             }
         }
-        if (src.count > kFusedSources) {
+        if (src.count > kCtaBounds) {
             if (!(ok = count_sync(g, sh.flag, nothing))) break;
             source_bound_pruned(m, blocks, s, src, p, cfl, first, stride);
         }
         auto control = [&] {
-            if (src.count && src.count <= kFusedSources) {
+            if (src.count && src.count <= kCtaBounds) {
                 source_bound_cta(m, s, src, p, cfl);
                 __syncthreads();  // the bounds land before step_control reads them
             }

@@ -38,14 +38,15 @@ namespace swe {
 // arrive while it computes its fluxes); a dense step spreads the queue over all
 // CTAs.
 //
-// Sources: up to kFusedSources of them cost a step no barrier of their own. The CTA
-// that computes a tile adds its sources right after the tile's corrector (each thread
-// looks at a few of the listed cells, which stay in L1), and the CFL bounds, which need
-// every neighbour's depth after its own source, are taken by the step control's CTA.
+// Sources: up to kFusedSources of them are added by the CTA that computes their tile,
+// right after the tile's corrector (each thread looks at a few of the listed cells,
+// which stay in L1). Their CFL bounds, which need every neighbour's depth after its own
+// source, are taken by the step control's CTA without a barrier of their own up to
+// kCtaBounds, and by a grid-wide pass behind one more barrier past that.
 // A source in an inactive block (whose committed depth correctors of neighbouring
 // tiles read) waits for one more barrier, in the steps that have one: the step control
-// says so in advance. More sources than that (rain) run as two grid-wide passes with
-// a barrier before each.
+// says so in advance. More sources than kFusedSources (rain) run as two grid-wide passes
+// with a barrier before each.
 //
 // Step control: the last CTA to arrive at a step's final barrier runs it for
 // every instance after the others have gone on, and publishes each instance's
@@ -612,6 +613,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
     uint32_t ph[2] = {0u, 0u};
     uint64_t computed = 0;
     const bool fused = src.count != 0u && src.count <= kFusedSources;
+    const bool by_cta = fused && src.count <= kCtaBounds;  // the step control's CTA takes the sources' bounds
     bool ok = true, idle = false;
     uint32_t step = 0;
     for (; step < n_steps; ++step) {
@@ -633,9 +635,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         if (src.count && !fused) {
             if (!(ok = count_sync(g, flag, nothing))) break;
             source_apply(m, s, src, p.dry_tol, COMP ? 1 : 0, first, stride);
+        }
+        if (src.count && !by_cta) {
             if (!(ok = count_sync(g, flag, nothing))) break;
             source_bound(m, s, src, p, cfl, first, stride);
-            if (!all) {  // a source that wets its block marks the block's two-ring
+            if (!fused && !all) {  // a source that wets its block marks the block's two-ring
                 for (uint32_t q = first; q < src.count; q += stride) {
                     const uint32_t b = src.cells[q] >> 8;
                     if (s.blk[kBlkWords * b + kBlkWet] != 0u && s.dt_buf[kDtWords * m.block_inst[b]] != 0u)
@@ -645,7 +649,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1024 / kPersistThreads)
         }
         const bool last_step = step + 1u == n_steps;
         auto control = [&] {
-            if (fused) {
+            if (by_cta) {
                 source_bound_cta(m, s, src, p, cfl);
                 __syncthreads();  // the bounds land before step_control reads them
             }

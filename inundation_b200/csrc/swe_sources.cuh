@@ -34,11 +34,17 @@ __device__ __forceinline__ float clock_seconds(const swe_ctrl_t *c) {
     return static_cast<float>(c->now_ticks) * (1.0f / kTicksPerSecond);
 }
 
-// Sources up to which the fused form is taken: at most four list entries per thread and tile, read from L1.
-// 540 steps of a 30k-cell mesh with 7 inflows take 7.0 ms this way; with the two grid-wide passes (two more
-// barriers a step, one thread following a source's slots and marking its two-ring one block after the
-// other) they took 16.9 ms, 28 us a step.
+// Sources that the persistent kernel's CTAs add with their tiles: at most four list entries per thread and tile, read
+// from L1. Past it every source is a thread's of a grid-wide pass, which needs a barrier, and marks its two-ring one block
+// after the other. A step of 30k cells with 1024 sources against 1025: 18.5 and 32.5 us (260k cells: 54 and 73 us).
 constexpr uint32_t kFusedSources = 1024;
+
+// Sources whose CFL bounds the step control's CTA takes, in the persistent and the dense kernel. It has 32 groups of
+// eight lanes, and a round of them is a chain of five dependent loads, some 3 us, that the whole grid waits for; a
+// grid-wide pass costs one barrier and one such chain. A persistent step of 30k cells with 64 sources: 15.0 us by the
+// CTA, with 65 17.7 us by the pass (with 256 and 1024: 25.6 and 65 us by the CTA, 18.2 and 18.5 by the pass); a dense
+// step of 260k cells: 64 24.9 us, 65 24.4 us (1024: 78 us by the CTA, 27 by the pass).
+constexpr uint32_t kCtaBounds = 64;
 
 // Source k's increment of cell i (of an instance whose step is dt), into the committed depth; keep != nullptr:
 // the cell's h also goes to keep[0] and its low word to keep[3 x 64] (a tile's state held in shared memory).
