@@ -31,7 +31,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import native
-from .engine import AUTO_DENSE_FRACTION, KERNELS, START, ResidentEngine
+from .engine import AUTO_DENSE_FRACTION, KERNELS, PERSISTENT_FUSED_SOURCES, START, ResidentEngine
 from .layout import build_tile_layout
 from .mesh.geometry import MeshGeometry
 from .sources import Hydrograph
@@ -64,7 +64,7 @@ class GaugeCalibration(ResidentEngine):
     stage_kernel: str = "tiled"
     packed_blocks: bool = False  # every step is one swe_step, and set_parameters moves the bed steps
     # run the forward in the persistent kernel, gauges included, while few blocks are active (as "auto"
-    # does); False, more blocks, or another stage kernel: graphs of the per-step kernels. The same bits.
+    # does); False, more blocks, many sources, or another stage kernel: graphs of the per-step kernels. The same bits.
     persistent_forward: bool = True
     # reverse each segment in one cooperative launch (grid barriers between phases) instead of one
     # launch per phase and step; the arithmetic is the same. Off by default: at 250k cells the
@@ -234,8 +234,10 @@ class GaugeCalibration(ResidentEngine):
         """``n_steps`` steps with the gauges after each, on the solver's stream."""
         grid = self.grid(KERNELS["persistent"])
         sparse = self._active_blocks <= AUTO_DENSE_FRACTION * self.n_blocks or 4 * self._active_blocks <= grid
+        # more sources than its tiles' CTAs add: rain on 250k cells took 98 ms for 200 steps, 17 ms in the graph
+        few = self._src_count <= PERSISTENT_FUSED_SOURCES
         if self.persistent_forward and self.stage_kernel == "tiled" and not self.track_clamp and self._persistent_fits \
-                and sparse:
+                and sparse and few:
             params, sources = self._params(), self._sources()
             params.kernel, params.grid = KERNELS["persistent"], grid
             native.check(

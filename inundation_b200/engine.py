@@ -52,7 +52,7 @@ KERNELS = {"tiled": 0, "plain": 1, "persistent": 2, "staged": 3}
 # whole GPU), unless every active tile still has a CTA of the persistent grid to itself (a small mesh).
 AUTO_DENSE_FRACTION = 0.25
 PERSISTENT_EXTRA_TILES = 512  # kExtraCap of the persistent kernel
-
+PERSISTENT_FUSED_SOURCES = 1024  # its kFusedSources
 DENSE_TAKEN_BLOCKS = 512  # kTakenCap of the dense whole-step kernel
 
 
