@@ -240,13 +240,13 @@ class GaugeCalibration(ResidentEngine):
                 and sparse and few:
             params, sources = self._params(), self._sources()
             params.kernel, params.grid = KERNELS["persistent"], grid
-            native.check(
-                self._lib.swe_steps_gauged(ctypes.byref(self._mesh), ctypes.byref(self._state), ctypes.byref(params),
-                                           ctypes.byref(sources), ctypes.byref(self._gauges), record, n_steps,
-                                           self._cuda_stream),
-                "swe_steps_gauged",
-            )
-            return
+            rc = self._lib.swe_steps_gauged(ctypes.byref(self._mesh), ctypes.byref(self._state), ctypes.byref(params),
+                                            ctypes.byref(sources), ctypes.byref(self._gauges), record, n_steps,
+                                            self._cuda_stream)
+            # the gauges' shared memory may leave fewer CTAs than grid() counts: refused before anything is launched
+            if rc != native.ERR_TOO_LARGE:
+                native.check(rc, "swe_steps_gauged")
+                return
         graph = self._segment_graph(n_steps, record)
         with torch.cuda.stream(self._stream):
             graph.replay()

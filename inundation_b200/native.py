@@ -14,6 +14,7 @@ from .build import LIB_PATH
 _P = ctypes.c_void_p
 _U32 = ctypes.c_uint32
 
+ERR_TOO_LARGE = 3  # SWE_ERR_TOO_LARGE
 STATUS_MESSAGES = {
     1: "invalid argument",
     2: "CUDA launch or runtime error",

@@ -1,7 +1,7 @@
 """Which kernel a calibration's forward segment takes, on a stub (no device).
 
 The persistent kernel where "auto" would take it and its tiles' CTAs add the sources themselves; graphs of the
-per-step kernels otherwise.
+per-step kernels otherwise, among them for a mesh that the gauged kernel's grid cannot hold (the library refuses it).
 """
 
 from __future__ import annotations
@@ -14,7 +14,7 @@ from inundation_b200 import native
 from inundation_b200.adjoint import GaugeCalibration
 from inundation_b200.engine import KERNELS, PERSISTENT_FUSED_SOURCES
 
-SWE_OK = 0
+SWE_OK, SWE_ERR_CUDA, SWE_ERR_TOO_LARGE = 0, 2, 3
 
 
 class Graph:
@@ -67,6 +67,12 @@ def test_the_active_blocks_decide_as_for_auto(active: int, n_blocks: int, want: 
 def test_many_sources_take_the_graph(sources: int, want: str) -> None:
     """Rain on every cell took six times as long in the persistent kernel (250k cells: 98 ms against 17)."""
     assert segment(50, sources=sources) == [want]
+
+
+def test_a_mesh_that_the_gauged_grid_cannot_hold_takes_the_graph() -> None:
+    assert segment(50, status=SWE_ERR_TOO_LARGE) == ["graph"]
+    with pytest.raises(RuntimeError, match="swe_steps_gauged"):
+        segment(50, status=SWE_ERR_CUDA)
 
 
 @pytest.mark.parametrize("attributes", [{"persistent_forward": False}, {"stage_kernel": "plain"}, {"track_clamp": True}])
