@@ -31,7 +31,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import native
-from .engine import AUTO_DENSE_FRACTION, KERNELS, PERSISTENT_FUSED_SOURCES, START, ResidentEngine
+from .engine import KERNELS, PERSISTENT_FUSED_SOURCES, START, ResidentEngine
 from .layout import build_tile_layout
 from .mesh.geometry import MeshGeometry
 from .sources import Hydrograph
@@ -63,8 +63,10 @@ class GaugeCalibration(ResidentEngine):
     # the segment graphs capture one swe_step per step: a per-step stage kernel
     stage_kernel: str = "tiled"
     packed_blocks: bool = False  # every step is one swe_step, and set_parameters moves the bed steps
-    # run the forward in the persistent kernel, gauges included, while few blocks are active (as "auto"
-    # does); False, more blocks, many sources, or another stage kernel: graphs of the per-step kernels. The same bits.
+    # run the forward in the persistent kernel, gauges included, where few blocks are active in the initial state
+    # ("auto"'s rule, looked at once a run: a look at every segment took water that spread from 24 % to 65 % of 120k
+    # cells off it, 40 ms instead of 30 for 1500 steps); False, more blocks, many sources, or another stage kernel:
+    # graphs of the per-step kernels. The same bits.
     persistent_forward: bool = True
     # reverse each segment in one cooperative launch (grid barriers between phases) instead of one
     # launch per phase and step; the arithmetic is the same. Off by default: at 250k cells the
@@ -232,14 +234,11 @@ class GaugeCalibration(ResidentEngine):
 
     def _forward_steps(self, n_steps: int, record: int) -> None:
         """``n_steps`` steps with the gauges after each, on the solver's stream."""
-        grid = self.grid(KERNELS["persistent"])
-        sparse = self._active_blocks <= AUTO_DENSE_FRACTION * self.n_blocks or 4 * self._active_blocks <= grid
         # more sources than its tiles' CTAs add: rain on 250k cells took 98 ms for 200 steps, 17 ms in the graph
         few = self._src_count <= PERSISTENT_FUSED_SOURCES
-        if self.persistent_forward and self.stage_kernel == "tiled" and not self.track_clamp and self._persistent_fits \
-                and sparse and few:
+        if self.persistent_forward and self.stage_kernel == "tiled" and not self.track_clamp and few and self._sparse:
             params, sources = self._params(), self._sources()
-            params.kernel, params.grid = KERNELS["persistent"], grid
+            params.kernel, params.grid = KERNELS["persistent"], self.grid(KERNELS["persistent"])
             rc = self._lib.swe_steps_gauged(ctypes.byref(self._mesh), ctypes.byref(self._state), ctypes.byref(params),
                                             ctypes.byref(sources), ctypes.byref(self._gauges), record, n_steps,
                                             self._cuda_stream)

@@ -221,14 +221,18 @@ class ResidentEngine:
     @property
     def _kernel(self) -> int:
         if self.stage_kernel == "auto":
-            dense = self._active_blocks > AUTO_DENSE_FRACTION * self.n_blocks
-            seated = 4 * self._active_blocks <= self.grid(KERNELS["persistent"])
-            if self._persistent_fits and (seated or not dense):
+            if self._sparse:
                 return KERNELS["persistent"]
             return KERNELS["staged"] if self._staged_fits else KERNELS["plain"]
         if self.stage_kernel not in KERNELS:
             raise ValueError(f"stage_kernel must be one of {sorted(KERNELS)} or 'auto', got {self.stage_kernel!r}")
         return KERNELS[self.stage_kernel]
+
+    @property
+    def _sparse(self) -> bool:
+        """Whether the active blocks, as last read, are few enough for the persistent kernel."""
+        seated = 4 * self._active_blocks <= self.grid(KERNELS["persistent"])
+        return self._persistent_fits and (seated or self._active_blocks <= AUTO_DENSE_FRACTION * self.n_blocks)
 
     @property
     def _persistent_fits(self) -> bool:
