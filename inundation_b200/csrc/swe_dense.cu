@@ -414,6 +414,9 @@ int swe_configure_blocks(const swe_mesh_t *mesh, const swe_blocks_t *blocks, int
     const size_t bytes = block_bytes(mesh, blocks);
     if (bytes > kMaxSmem || kBlockCells + blocks->max_halo >= kNoCell || mesh->max_tile_edges > 32u * kThreads)
         return SWE_OK;
+    cudaFuncAttributes own;
+    if (cudaFuncGetAttributes(&own, dense_steps_kernel<true, false, false>) != cudaSuccess) return SWE_ERR_CUDA;
+    if (bytes + own.sharedSizeBytes > kMaxSmem) return SWE_OK;
     const int rc = set_smem(dense_steps_kernel<true, false, false>, bytes);
     if (rc) return rc;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, dense_steps_kernel<true, false, false>, kThreads,
