@@ -178,18 +178,13 @@ class ResidentEngine:
     def _pack_blocks(self, t: dict[str, torch.Tensor], B: TileSet) -> None:
         """The 256-cell tiles' records as the dense whole-step kernel reads them, packed on the device from the
         uploaded arrays: (nx, ny, len, local cells) and (dzl, dzr) side by side."""
-        self._blocks = None
+        self._blocks, self._blocks_t = None, {}
         if not self._staged_fits or not self.packed_blocks:
             return
         H = halo_records(B, t["tile_cl"], t["tile_cr"], self.layout.n_padded_cells)
         if B.tile_cells + H.max_halo >= NO_CELL:
             return  # a local index has 16 bits
-        self._blocks_t = {
-            "rec": torch.stack([t["tile_nx"], t["tile_ny"], t["tile_len"], H.local.view(torch.float32)], dim=1),
-            "dz": torch.stack([t["tile_dzl"], t["tile_dzr"]], dim=1),
-            "halo": H.halo, "halo_ptr": H.halo_ptr,
-        }
-        dz = self._blocks_t["dz"]
+        dz = torch.stack([t["tile_dzl"], t["tile_dzr"]], dim=1)
         if not bool(((dz >= 0.0) & (dz <= 2.0**19)).all()):
             return  # not the face steps of a bed: the kernel's range check relies on them
         # every cell's perimeter, rounded up by more than the order of summing its edges can change
@@ -199,14 +194,17 @@ class ResidentEngine:
         length = t["tile_len"].double()
         around.index_add_(0, t["tile_cl"], torch.where(own, length, 0.0))
         around.index_add_(0, t["tile_cr"].clamp(min=0), torch.where(inner, length, 0.0))
-        self._blocks_t["perim"] = (around * (1.0 + 1e-4)).float()
-        blocks = native.SweBlocks(max_halo=H.max_halo, **{k: v.data_ptr() for k, v in self._blocks_t.items()})
+        packed = {
+            "rec": torch.stack([t["tile_nx"], t["tile_ny"], t["tile_len"], H.local.view(torch.float32)], dim=1),
+            "dz": dz, "halo": H.halo, "halo_ptr": H.halo_ptr, "perim": (around * (1.0 + 1e-4)).float(),
+        }
+        blocks = native.SweBlocks(max_halo=H.max_halo, **{k: v.data_ptr() for k, v in packed.items()})
         per_sm = ctypes.c_int(0)
         with torch.cuda.device(self.device):
             native.check(self._lib.swe_configure_blocks(ctypes.byref(self._mesh), ctypes.byref(blocks),
                                                         ctypes.byref(per_sm)), "swe_configure_blocks")
         if per_sm.value > 0:
-            self._blocks, self._dense_per_sm = blocks, per_sm.value
+            self._blocks, self._blocks_t, self._dense_per_sm = blocks, packed, per_sm.value
 
     def grid(self, kernel: int | None = None) -> int:
         """Persistent CTAs of a stage kernel: CTAs per SM x SMs, at most one per work unit."""
