@@ -117,6 +117,7 @@ class ResidentEngine:
         self._cfl = float(self.default_cfl if cfl is None else cfl)
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         self._stream = torch.cuda.Stream(device=self.device)
+        self._src_host: list | None = None
         self._upload_mesh(layout, n_mann)
         self._alloc_state()
         self._graphs: dict[tuple, torch.cuda.CUDAGraph] = {}
@@ -171,16 +172,29 @@ class ResidentEngine:
             self._per_sm[kernel] = max(1, per_sm.value)
             if kernel == KERNELS["staged"]:  # 0: the mesh's largest block does not fit its shared memory
                 self._staged_fits = per_sm.value > 0
-        self._pack_blocks(t, B)
         self.ctas_per_sm: int | None = None  # None: as many as fit
         self.max_grid: int | None = None  # an upper bound on the persistent CTAs (None: none)
+        self._blocks, self._blocks_t = None, {}
+        self._packing_tried = False
+        # A mesh whose every tile has a CTA of the persistent kernel never leaves it in "auto": its records are packed
+        # when "staged" is asked for (at 8k cells the packing made a construction 9.0 instead of 7.5 ms, the first of a process 300 instead of 50).
+        if 4 * L.n_blocks > self.grid(KERNELS["persistent"]):
+            self._packed()
+
+    def _packed(self) -> native.SweBlocks | None:
+        """The packed records, made when first asked for (None: not wanted, or not for this mesh)."""
+        if not self.packed_blocks or not self._staged_fits:
+            return None
+        if not self._packing_tried:
+            self._packing_tried = True
+            self._pack_blocks(self._mesh_t, self.layout.blocks)
+            self._set_block_sources()
+            torch.cuda.current_stream(self.device).synchronize()  # the solver's stream reads them
+        return self._blocks
 
     def _pack_blocks(self, t: dict[str, torch.Tensor], B: TileSet) -> None:
         """The 256-cell tiles' records as the dense whole-step kernel reads them, packed on the device from the
         uploaded arrays: (nx, ny, len, local cells) and (dzl, dzr) side by side."""
-        self._blocks, self._blocks_t = None, {}
-        if not self._staged_fits or not self.packed_blocks:
-            return
         H = halo_records(B, t["tile_cl"], t["tile_cr"], self.layout.n_padded_cells)
         if B.tile_cells + H.max_halo >= NO_CELL:
             return  # a local index has 16 bits
@@ -347,17 +361,14 @@ class ResidentEngine:
         host = [np.asarray(cells, np.int64), np.asarray(rate, np.float32),
                 None if hidx is None else np.asarray(hidx), None if hscale is None else np.asarray(hscale),
                 [(np.asarray(t, np.float32), np.asarray(q, np.float32)) for t, q in knots]]
-        if getattr(self, "_src_host", None) is not None and _same_sources(self._src_host, host):
+        if self._src_host is not None and _same_sources(self._src_host, host):
             return
         self._src_host = host
         dev = self._dev
         self._src_count = int(cells.size)
         self._src_cells = dev(cells.astype(np.int32) if cells.size else np.zeros(1, np.int32))
         self._src_rate = dev(rate.astype(np.float32) if cells.size else np.zeros(1, np.float32))
-        if self._blocks is not None:  # the sources of every block, by ascending cell
-            bounds = np.arange(self.n_blocks + 1) * ACTIVE_BLOCK_CELLS
-            self._src_ptr = dev(np.searchsorted(host[0], bounds).astype(np.int32)) if self._src_count else None
-            self._blocks.src_ptr = self._src_ptr.data_ptr() if self._src_count else None
+        self._set_block_sources()
         self._src_hydro = None
         if hidx is not None and knots:
             ptr = np.zeros(len(knots) + 1, np.int64)
@@ -371,6 +382,16 @@ class ResidentEngine:
                 "n": len(knots),
             }
         self._src_version += 1
+
+    def _set_block_sources(self) -> None:
+        """The sources of every packed block, by ascending cell."""
+        if self._blocks is None:
+            return
+        cells = np.zeros(0, np.int64) if self._src_host is None else self._src_host[0]
+        if cells.size:
+            bounds = np.arange(self.n_blocks + 1) * ACTIVE_BLOCK_CELLS
+            self._src_ptr = self._dev(np.searchsorted(cells, bounds).astype(np.int32))
+        self._blocks.src_ptr = self._src_ptr.data_ptr() if cells.size else None
 
     def _sources(self) -> native.SweSources:
         s = native.SweSources(cells=self._src_cells.data_ptr(), rate=self._src_rate.data_ptr(), count=self._src_count)
@@ -540,7 +561,7 @@ class ResidentEngine:
         steps = self.steps_per_graph if steps is None else steps
         if self._kernel == KERNELS["persistent"]:
             return _PersistentSubmit(self, steps)
-        if self._kernel == KERNELS["staged"] and self._blocks is not None:
+        if self._kernel == KERNELS["staged"] and self._packed() is not None:
             submit = _DenseSubmit(self, steps)
             if submit.fits:
                 return submit

@@ -9,11 +9,11 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from inundation_b200.engine import _DenseSubmit
+from inundation_b200.engine import KERNELS, _DenseSubmit
 from inundation_b200.mesh.geometry import with_bed
 from oracle.resident_oracle import ResidentOracle
 
-from ._valley import MANNING, dam, valley_grid
+from ._valley import MANNING, dam, point_source, valley_grid
 
 pytestmark = pytest.mark.gpu
 
@@ -39,6 +39,29 @@ def same_run(a, b, **kw) -> None:
     for name in ("h", "hu", "hv", "h_residual"):
         p, q = getattr(a, f"download_{name}")(), getattr(b, f"download_{name}")()
         np.testing.assert_array_equal(p.view(np.uint32), q.view(np.uint32), err_msg=name)
+
+
+def test_a_mesh_that_is_always_seated_is_packed_when_asked_for() -> None:
+    """512 tiles have a CTA each: "auto" never leaves the persistent kernel, so nothing is packed until "staged" is
+    chosen; the sources set before that come along."""
+    grid = valley_grid()
+    solver, oracle = solver_of(grid, dam(grid)), oracle_of(grid, dam(grid))
+    assert 4 * solver.n_blocks <= solver.grid(KERNELS["persistent"])
+    assert solver._blocks is None and not solver._blocks_t
+    src = point_source(grid, 0.5, 60.0, 128.0)
+    same_run(solver, oracle, source_rate=src)
+    assert solver._blocks is None
+    solver.stage_kernel = "staged"
+    assert isinstance(solver._graph(), _DenseSubmit) and solver._blocks is not None
+    solver.steps_total = oracle.steps_total = 0
+    same_run(solver, oracle, source_rate=src)
+
+
+def test_a_larger_mesh_is_packed_at_once() -> None:
+    geom = valley_grid(nx=256, ny=256)
+    solver = solver_of(geom, dam(geom, ny=256))
+    assert 4 * solver.n_blocks > solver.grid(KERNELS["persistent"])
+    assert solver._blocks is not None
 
 
 def test_bed_steps_out_of_range_leave_no_records_behind() -> None:
