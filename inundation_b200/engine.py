@@ -177,7 +177,8 @@ class ResidentEngine:
         self._blocks, self._blocks_t = None, {}
         self._packing_tried = False
         # A mesh whose every tile has a CTA of the persistent kernel never leaves it in "auto": its records are packed
-        # when "staged" is asked for (at 8k cells the packing made a construction 9.0 instead of 7.5 ms, the first of a process 300 instead of 50).
+        # when "staged" is asked for (at 8k cells the packing made a construction 9.0 instead of 7.5 ms, the first of a
+        # process 300 instead of 50).
         if 4 * L.n_blocks > self.grid(KERNELS["persistent"]):
             self._packed()
 

@@ -25,13 +25,13 @@ def solver_of(geom, h0, **kw):
     return SWESolverB200Resident(geom, None, h0, z, z, n, **kw)
 
 
-def oracle_of(geom, h0):
+def oracle_of(geom, h0, **kw):
     z, n = np.zeros(geom.N, np.float32), np.full(geom.N, MANNING, np.float32)
-    return ResidentOracle(geom, h0, z, z, n)
+    return ResidentOracle(geom, h0, z, z, n, **kw)
 
 
 def same_run(a, b, **kw) -> None:
-    run = dict(t_end=2.0, output_interval_s=0.5, dt_max=0.5, dt_init=0.01, cfl_interval=1, progress=False, **kw)
+    run = {**dict(t_end=2.0, output_interval_s=0.5, dt_max=0.5, dt_init=0.01, cfl_interval=1, progress=False), **kw}
     x, _ = a.run(**run)
     y, _ = b.run(**run)
     assert a.steps_total == b.steps_total
