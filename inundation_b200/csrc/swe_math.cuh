@@ -203,10 +203,13 @@ __device__ __forceinline__ void wall_mirror(float huL, float hvL, float nx, floa
 // rsqrt.approx, about one ulp) by Newton steps in fused multiply-adds, ended by the correction
 // that Markstein proved to round correctly (P. Markstein, "Computation of elementary functions
 // on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: from the correctly rounded
-// reciprocal y of b and a quotient q within one ulp, fma(fma(-b, q, a), y, q) is the correctly
-// rounded a / b; likewise for the root with half its reciprocal). They equal the IEEE operations
-// for operands far from under- and overflow, which the caller checks: x and b in [2^-80, 2^62],
-// a quotient's numerator 0 or in that range (a zero quotient may come out with the other sign).
+// reciprocal y of b and a quotient q near a / b, fma(fma(-b, q, a), y, q) is the correctly
+// rounded a / b; likewise for the root with half its reciprocal). The product a y that stands for q
+// can be 1.5 ulp off, half an ulp more than the theorem allows, when a < b: the quotients nearest to
+// a rounding boundary (the 15 numerators on either side, for every mantissa of b) all round right.
+// They equal the IEEE operations for operands far from under- and overflow, which the caller checks:
+// b and a root's x in [2^-80, 2^62], a root's x also down to 2^-96, a quotient's numerator 0 or in
+// that range (a zero quotient may come out with the other sign).
 // The compiler's own operations check every operand and branch, so several in a row cannot
 // overlap; these can, and two of a kind share the paired instructions.
 constexpr float kPlainMin = 8.271806125530277e-25f;  // 2^-80

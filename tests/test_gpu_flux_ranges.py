@@ -53,3 +53,24 @@ def test_states_outside_the_plain_range(case: str, kernel: str) -> None:
         x, y = getattr(solver, f"download_{name}")(), getattr(oracle, f"download_{name}")()
         same = (x.view(np.uint32) == y.view(np.uint32)) | (np.isnan(x) & np.isnan(y))
         assert same.all(), (name, int((~same).sum()), x[~same][:3], y[~same][:3])
+
+
+@pytest.mark.parametrize("kernel", ["persistent", "staged", "tiled"])
+def test_films_under_the_smallest_gravity_of_the_plain_range(kernel: str) -> None:
+    """Depths from 2^-100 to 2^-60 and a gravity just above 1/16: celerity arguments down to 2^-85 and below."""
+    from inundation_b200.backend import SWESolverB200Resident
+
+    grid = valley_grid(nx=64, ny=48)
+    rng = np.random.default_rng(12)
+    h = np.where(rng.random(grid.N) < 0.2, 0.01, 2.0 ** rng.uniform(-100, -60, grid.N)).astype(np.float32)
+    z, n, kw = np.zeros(grid.N, np.float32), np.full(grid.N, MANNING, np.float32), {"g": 0.07, "dry_tol": 1e-9}
+    solver, oracle = SWESolverB200Resident(grid, None, h, z, z, n, **kw), ResidentOracle(grid, h, z, z, n, **kw)
+    solver.stage_kernel = kernel
+    t = 2.0**-6
+    for s in (solver, oracle):
+        s.steps_per_graph = 20
+        s.run(t_end=t, output_interval_s=t, dt_max=t / 16, dt_init=t / 16, cfl_interval=1, progress=False)
+    assert solver.steps_total == oracle.steps_total >= 16
+    for name in ("h", "hu", "hv", "h_residual"):
+        x, y = getattr(solver, f"download_{name}")(), getattr(oracle, f"download_{name}")()
+        np.testing.assert_array_equal(x.view(np.uint32), y.view(np.uint32), err_msg=name)
