@@ -278,6 +278,22 @@ def plan(solver, sc) -> None:
     solver._read_ctrl()
 
 
+def kernel_launches(submit, steps: int, sources: int) -> int:
+    """Kernels that one submit of ``steps`` steps launches: one cooperative launch of whole steps (the dense kernel's is
+    followed by its hand-over), or in every step two stages, the dilation and what the sources take."""
+    from inundation_b200.engine import FEW_SOURCES, _DenseSubmit, _PersistentSubmit
+
+    if isinstance(submit, _PersistentSubmit):
+        return 2 if isinstance(submit, _DenseSubmit) else 1
+    return steps * (3 + (0 if sources == 0 else 1 if sources <= FEW_SOURCES else 2))
+
+
+def submits(solver, steps: int, per_submit: int) -> list[tuple[object, int]]:
+    """The submits of ``steps`` steps, ``per_submit`` at a time, each with its steps."""
+    full, rest = divmod(steps, per_submit)
+    return [(solver._graph(per_submit), per_submit)] * full + ([(solver._graph(rest), rest)] if rest else [])
+
+
 def capture_chunks(solver, steps: int, chunk: int, timed: bool):
     """Graphs covering exactly ``steps`` steps; with ``timed``, events around every stage launch."""
     import ctypes
@@ -289,12 +305,7 @@ def capture_chunks(solver, steps: int, chunk: int, timed: bool):
     graphs, events = [], []
     if solver.stage_kernel in ("persistent", "staged"):
         # one cooperative launch of whole steps per chunk; its phases are not separate launches to time
-        left = steps
-        while left > 0:
-            n = min(chunk, left)
-            left -= n
-            graphs.append(solver._graph(n))
-        return graphs, events
+        return [submit for submit, _ in submits(solver, steps, chunk)], events
     params, sources = solver._params(), solver._sources()
     mesh, state = ctypes.byref(solver._mesh), ctypes.byref(solver._state)
     left = steps
@@ -379,6 +390,7 @@ def forward_line(args, sc, world: int, local: int):
     import torch
 
     from inundation_b200.backend import SWESolverB200Resident
+    from inundation_b200.engine import _PersistentSubmit
     from inundation_b200.layout import algorithmic_bytes_per_cell_step
 
     device = f"cuda:{local}"
@@ -442,7 +454,10 @@ def forward_line(args, sc, world: int, local: int):
         for k in range(n):
             stage_ms += ev[3 * k].elapsed_time(ev[3 * k + 1]) + ev[3 * k + 1].elapsed_time(ev[3 * k + 2])
             dilate_ms += ev[3 * k + 2].elapsed_time(ev[3 * k + 3])
-    launches = 2 * args.steps if events else len(graphs)
+    whole = isinstance(graphs[0], _PersistentSubmit)  # whole steps, one launch a chunk
+    launches = len(graphs) if whole else 2 * args.steps
+    per_graph = [args.chunk] * (args.steps // args.chunk) + [args.steps % args.chunk]
+    gpu_launches = sum(kernel_launches(g_, n, solver._src_count) for g_, n in zip(graphs, per_graph))
     bpc = algorithmic_bytes_per_cell_step(g)
     alg_bytes = computed * bpc  # over all stage launches of the timed region
     achieved = alg_bytes / (stage_ms * 1e-3) / 1e9
@@ -472,7 +487,7 @@ def forward_line(args, sc, world: int, local: int):
         "computed_cell_steps_per_s": world * computed / (ms_max * 1e-3),
         "active_fraction": computed / (g.N * args.steps),
         "simulated_s": t_sim,
-        "gpu_launches": 3 * args.steps if events else len(graphs),
+        "gpu_launches": gpu_launches,
         "roofline": {
             "bound": "hbm",
             "achieved": achieved,
@@ -481,7 +496,7 @@ def forward_line(args, sc, world: int, local: int):
             "frac": achieved / peak,
             "traffic": traffic,
             "kernel": f"stage kernel, {args.kernel} (fused edge flux + gather + Heun update), both stages"
-            if events else f"{'persistent' if args.kernel == 'persistent' else 'dense'} step kernel (whole steps: both "
+            if not whole else f"{'persistent' if args.kernel == 'persistent' else 'dense'} step kernel (whole steps: both "
             "stages, dilation, step control; grid barriers)",
             "algorithmic_bytes_per_cell_step": bpc,
             "launches": launches,
@@ -838,7 +853,7 @@ def run_sources_workload(args, world: int, rank: int, local: int, built=None) ->
     import torch
 
     from inundation_b200.batch import BatchedSolver, BatchMember
-    from inundation_b200.engine import KERNELS
+    from inundation_b200.engine import KERNELS, _PersistentSubmit
     from inundation_b200.layout import algorithmic_bytes_per_cell_step
 
     device = f"cuda:{local}"
@@ -886,8 +901,9 @@ def run_sources_workload(args, world: int, rank: int, local: int, built=None) ->
     bpc = algorithmic_bytes_per_cell_step(g)
     peak, peak_kind = peaks()
     achieved = computed * bpc / (ms * 1e-3) / 1e9
-    whole = kernel in ("persistent", "staged")  # one cooperative launch of whole steps per chunk
-    stage_launches = 2 * args.steps if not whole else -(-args.steps // args.chunk)
+    done_by = submits(solver, args.steps, args.chunk)
+    whole = isinstance(done_by[0][0], _PersistentSubmit)  # whole steps, one launch a chunk
+    stage_launches = len(done_by) if whole else 2 * args.steps
     traffic = None
     tfile = ROOT / "profiles" / "stage_kernel_traffic.json"
     if tfile.exists():
@@ -929,7 +945,7 @@ def run_sources_workload(args, world: int, rank: int, local: int, built=None) ->
         "computed_cell_steps_per_s": world * computed / (ms_max * 1e-3),
         "active_fraction": computed / (g.N * args.steps),
         "simulated_s": t_sim,
-        "gpu_launches": stage_launches if whole else 5 * args.steps,  # stages, sources (2), dilation
+        "gpu_launches": sum(kernel_launches(submit, n, solver._src_count) for submit, n in done_by),
         "roofline": {
             "bound": "hbm",
             "achieved": achieved,
@@ -987,8 +1003,7 @@ def _timed_steps(solver, steps: int, graph_steps: int) -> float:
     import torch
 
     solver.steps_per_graph = graph_steps
-    full, rest = divmod(steps, graph_steps)
-    graphs = ([solver._graph()] * full) + ([solver._graph(rest)] if rest else [])
+    graphs = [submit for submit, _ in submits(solver, steps, graph_steps)]
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     torch.cuda.synchronize()
     with torch.cuda.stream(solver._stream):
@@ -1054,9 +1069,7 @@ def run_batch(args, world: int, local: int) -> dict:
         raise RuntimeError("batched end-to-end run stalled")
     del finals
     kernel = solver.stage_kernel
-    # stages, dilation (+ source increments and bounds), or one launch of whole steps for every 200
-    launches_per_step = 3 + (2 if solver._src_count else 0)
-    launches = -(-steps // 200) if kernel in ("persistent", "staged") else launches_per_step * steps
+    launches = sum(kernel_launches(submit, n, solver._src_count) for submit, n in submits(solver, steps, 200))
     del solver
     torch.cuda.empty_cache()
 

@@ -53,6 +53,7 @@ KERNELS = {"tiled": 0, "plain": 1, "persistent": 2, "staged": 3}
 AUTO_DENSE_FRACTION = 0.25
 PERSISTENT_EXTRA_TILES = 512  # kExtraCap of the persistent kernel
 PERSISTENT_FUSED_SOURCES = 1024  # its kFusedSources
+FEW_SOURCES = 128  # kFewSources of swe_apply_sources: one launch, more take two
 DENSE_TAKEN_BLOCKS = 512  # kTakenCap of the dense whole-step kernel
 
 

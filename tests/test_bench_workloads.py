@@ -70,3 +70,16 @@ def test_reference_arm_states_the_cuda_arms_config(capsys: pytest.CaptureFixture
     assert line["config"] == json.loads(json.dumps(bench.workload_config(sc, args, 0.8)))
     assert line["impl"] == "reference" and line["cpu_baseline"]["kind"] == "port"
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["value"] > 0
+
+
+@pytest.mark.parametrize(
+    ("submit", "steps", "sources", "want"),
+    [("_PersistentSubmit", 200, 7, 1), ("_DenseSubmit", 200, 0, 2), ("graph", 200, 0, 600), ("graph", 50, 1, 200),
+     ("graph", 50, 128, 200), ("graph", 50, 129, 250)],
+)
+def test_launches_are_counted_from_what_was_submitted(submit: str, steps: int, sources: int, want: int) -> None:
+    """Not from the kernel's name: "staged" may run whole steps or stage by stage."""
+    from inundation_b200 import engine
+
+    made = object() if submit == "graph" else getattr(engine, submit).__new__(getattr(engine, submit))
+    assert bench.kernel_launches(made, steps, sources) == want
