@@ -3,11 +3,12 @@
 Every instance (its own mesh, bed, roughness, initial state and sources)
 takes whole 256-cell blocks of one concatenated layout
 (``layout.build_batch_layout``) and keeps its own integer clock, dt and CFL
-bound on the device. One step of the batch is one launch of each kernel over
-the active tiles of all instances together, so many small meshes fill the
-GPU that one alone would leave mostly idle; a CUDA graph holds
-``steps_per_graph`` such steps. An instance whose window is done runs no-op
-steps until the others finish.
+bound on the device. A step of the batch computes the active tiles of all
+instances together, so many small meshes fill the GPU that one alone would
+leave mostly idle. ``steps_per_graph`` steps are one submit: a cooperative
+launch of whole steps, or a CUDA graph of the per-step kernels, as the stage
+kernel has it. An instance whose window is done runs no-op steps until the
+others finish.
 
 Each instance's results are bit-identical to a run of that scenario alone
 (same tiles, same gather order, its own dt), which the tests check.

@@ -590,8 +590,9 @@ __global__ void __launch_bounds__(kThreads)
 
 // The edge phases are bound by latency: a chain of loads (list, tile, records, states), then some 25 IEEE quotients
 // in turn per edge (shared reciprocals would take 14 and 10 us instead of 21 and 16, but move the knots' float64
-// gradients by 1e-7). 64 registers let 592 CTAs be resident, one tile each at 250k cells with 14 % active, where
-// 100 registers took two rounds: edge<1> with the predictor's cell update 27.2 -> 21.3 us, edge<0> 20.9 -> 16.3 us.
+// gradients by 1e-7). 64 registers let 592 CTAs be resident, one tile each at 250k cells with 14 % active, at the price
+// of 36 and 12 spilled bytes; without the bound they take 100 and the tiles two rounds: edge<1> with the predictor's
+// cell update 21.3 us instead of 27.2, edge<0> 16.3 instead of 20.9.
 constexpr int kAdjEdgeCtas = 4;
 
 template <int STAGE>

@@ -1,6 +1,6 @@
 // One Heun stage of a 256-cell block from packed records (the dense whole-step kernel).
 //
-// A dense step is bound by instruction issue, not by bytes, so a block's work is
+// A dense step is bound by issue and barriers, not by bytes, so a block's work is
 // laid out for few instructions per edge:
 //   * the velocities of every cell the block's edges read (its own and its halo
 //     list's) are computed once, by one thread per cell, into float4 (h, u, v, inv)
@@ -15,7 +15,7 @@
 //     that starts at +0 is never -0, and adding either zero to it changes nothing.
 // The records, the CSR pointers and the local CSR arrive by bulk copies on one
 // mbarrier while the threads load the cells' states.
-// A stage of 256 cells executes 1540 warp instructions per 32 cells this way.
+// A stage executes 1534 warp instructions per 32 cells this way (a million wet cells, 20 steps).
 #pragma once
 
 #include "swe_tiled.cuh"

@@ -19,10 +19,12 @@
 // to kCtaBounds sources are taken by the step control's CTA; those of more by a pass over all of them
 // after a barrier, which looks only at the cells whose bound can be below the smallest one so far:
 // a source's wave speeds are at most u + 2c on its whole perimeter.
-// Bound: instruction issue (a steady 75-80 % of the slots; DRAM and L2 stay below 20 % of their peaks), then a
-// phase's last microseconds. Measured, one step (staged stage kernels and dilation before -> now): 600k cells
-// all wet 105 -> 81 us, 260k cells 44 % active 33.5 -> 21.5 us. With blocks dealt to CTAs in turn instead of taken, a phase of the first waits 15 us for
-// its last CTA (49 us instead of 41.7), and one of the second takes 16 us instead of 13.
+// Bound: issue and the waits at CTA barriers. Over a launch of 20 steps of a million wet cells 63 % of the issue slots
+// are used, and of the 12.7 cycles between two instructions of a warp 3.4 are waits at a CTA barrier (three or four a
+// block, one buffer per CTA), 2.1 for loads, 1.7 fixed latencies and 1.5 not selected; DRAM moves 285 B per cell and
+// step, 33 % of the copy bandwidth. One step: 600k cells all wet 81 us, 260k cells 44 % active 21.5 us (as two staged
+// stage kernels and a dilation 105 and 33.5 us). With blocks dealt to CTAs in turn instead of taken, a phase of the
+// first waits 15 us for its last CTA (49 us instead of 41.7), and one of the second takes 16 us instead of 13.
 //
 // Every barrier and staged-data wait is bounded, as in the other kernels. The results
 // are the other kernels' bit for bit: the same expressions, the same blocks active.
@@ -37,7 +39,7 @@
 namespace swe {
 
 // CTAs an SM must hold: with 4, 64 registers a thread and no spills (600k cells all wet 80.7 us a step, 260k cells
-// 44 % active 21.2); with 5, 48 registers (82.7 and 22.5); 6 spill more than the warps bring.
+// 44 % active 21.2); with 5, 48 registers (82.7 and 22.5); with 6 they spill.
 constexpr int kDenseMinCtas = 4;
 
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu;

@@ -190,9 +190,9 @@ __device__ __forceinline__ void safe_vel_pair(const Phys &p, float2 h, float2 in
     if (!(h.y > p.dry_tol)) v1.y = v2.y = 0.0f;
 }
 
-// The operations of the flux: IEEE, or the branch-free ones equal to them on plain operands (swe_math.cuh). A
-// step (before -> now): 8k-cell lake 9.5 -> 9.0 us, 1M-cell dam break 12.0 -> 11.6, 600k cells all wet 83.3 -> 81.
-// The range check costs about a third of what the operations save, so the dense kernel checks per cell.
+// The operations of the flux: IEEE, or the branch-free ones equal to them on plain operands (swe_math.cuh). A step
+// with the IEEE ones and with the others: 8k-cell lake 9.5 and 9.0 us, 1M-cell dam break 12.0 and 11.6, 600k cells all
+// wet 83.3 and 81. The range check costs about a third of what they save, so the dense kernel checks per cell.
 struct IeeeOps {
     static constexpr bool kPlain = false;
     __device__ static float rcp(float b) { return 1.0f / b; }
@@ -586,7 +586,8 @@ __device__ __forceinline__ bool tile_compute(const swe_mesh_t &m, const swe_stat
     const SideWords S{reinterpret_cast<float *>(B.cr), reinterpret_cast<float *>(B.cl), capE};
 
     // Edge fluxes; the edges whose operands are out of the branch-free operations' range once more after the loop.
-    // An open mesh's take the IEEE operations: with the ghosts' flux both kinds spill (12.7 against 11.5 us a step).
+    // An open mesh's take the IEEE operations: with the ghosts' flux the loop for both kinds spills (a channel's step
+    // 12.7 us instead of 11.5).
     if (OPEN) {
         for (uint32_t j = tid; j < it.ne; j += TPB) tile_edge<STAGE, OPEN, IeeeOps>(m, s, p, B, S, F, C0, base, j, dt);
     } else {

@@ -50,6 +50,10 @@ KERNELS = {"tiled": 0, "plain": 1, "persistent": 2, "staged": 3}
 # "auto": the persistent kernel while few blocks are active (its phases are latency-bound), the
 # staged 256-cell block kernel once more than this fraction of blocks is active (work for the
 # whole GPU), unless every active tile still has a CTA of the persistent grid to itself (a small mesh).
+# us a step, persistent and staged, at 260k cells: 20 % active 17.8 and 18.3, 28 % 20.5 and 19.7, 50 % 42 and 23; at
+# 120k 27 % 11.2 and 19.9, 50 % 19.5 and 20.4, 74 % 31 and 22; at 600k 8 % 18.2 and 22.6, 14 % 30 and 24. The line
+# between them lies near 240 active blocks at every size, a quarter of them at 260k cells: smaller meshes leave the
+# persistent kernel early, larger ones late (the fraction is from before the staged kernel ran whole steps).
 AUTO_DENSE_FRACTION = 0.25
 PERSISTENT_EXTRA_TILES = 512  # kExtraCap of the persistent kernel
 PERSISTENT_FUSED_SOURCES = 1024  # its kFusedSources
@@ -589,8 +593,9 @@ class ResidentEngine:
 
     @contextlib.contextmanager
     def _capture(self, graph: torch.cuda.CUDAGraph) -> Iterator[None]:
-        """Capture what the body enqueues on the solver's stream. Nothing is allocated in it, so the garbage
-        collection and the emptied allocator cache of ``torch.cuda.graph`` (10 ms and more on a first pass) are left out."""
+        """Capture what the body enqueues on the solver's stream. Nothing is allocated in it, so the synchronisation of
+        the whole device and the emptied allocator caches of ``torch.cuda.graph`` (10 ms and more on a first pass) are
+        left out."""
         self._stream.synchronize()
         with torch.cuda.stream(self._stream):
             graph.capture_begin()
